@@ -204,6 +204,20 @@ struct Problem {
   // (terms per pixel) x max |entry|, and the per-call max |u| (as bits)
   double mf_kbound = 0.0;
   DevBuf<unsigned long long> mf_umax;
+  // matrix-free walks (dda.cuh): row-major copies of the image (solver FP32,
+  // operator FP64), and of the fixed-point sums
+  DevBuf<float> x32t;
+  DevBuf<double> x64t;
+  DevBuf<long long> fxt;
+  DevBuf<int> slow_rays;   // rays traced outside the walks (dda_slow)
+  int nslow = 0;
+  DevBuf<double> slow_y;   // their row sums, indexed by ray
+  // pixel-driven back projection (gather.cuh), when the geometry allows it
+  bool par_ok = false;
+  DevBuf<double> par_ang;  // nA ParAngle records
+  DevBuf<double> par_fix;  // par_nfix ParFix records
+  int par_nfix = 0;
+  double par_s0 = 0, par_D = 1;
 
   cudaStream_t stream = nullptr;
 

@@ -23,11 +23,12 @@
 #include "spmv.cuh"
 #include "stream.cuh"
 #include "ncp.cuh"
-#include "trace.cuh"
+#include "gather.cuh"
 
 namespace airt {
 
 void mf_backproject_f32(Problem &P, const float *u, double *g64, const int *stop_flag);
+ParGather par_gather_of(const Problem &P);
 
 namespace {
 
@@ -95,6 +96,25 @@ __device__ __forceinline__ void flush(SirtState *st, Acc4 &a) {
   }
 }
 
+// flush without a block barrier: one warp's sums.
+template <bool ME>
+__device__ __forceinline__ void flush_warp(SirtState *st, Acc4 &a) {
+  const double r2 = warp_sum(a.r2), rmr = warp_sum(a.rmr);
+  double p2 = 0, pr = 0;
+  if (ME) {
+    p2 = warp_sum(a.p2);
+    pr = warp_sum(a.pr);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&st->acc[0], r2);
+    atomicAdd(&st->acc[1], rmr);
+    if (ME) {
+      atomicAdd(&st->acc[2], p2);
+      atomicAdd(&st->acc[3], pr);
+    }
+  }
+}
+
 __device__ __forceinline__ bool stopped(const SirtState *st) {
   return *(volatile const int *)&st->stop != 0;
 }
@@ -129,43 +149,73 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamCtasPerSm)
   flush<ME>(o.st, a);
 }
 
-// 12 resident 64-thread blocks per SM (80 registers, 40-90 bytes of spills):
-// the tracer is issue and latency bound, and 24 warps per SM ran C2 3 %
-// faster than the 20 that 96 registers allow.
+// r = b - A*x over sphericaltomo's circles, one thread per circle.
 template <bool ME>
-__global__ void __launch_bounds__(64, 12)
+__global__ void __launch_bounds__(64)
     k_sirt_fwd_mf(RayGeom g, int64_t nrays, bool excl, const float *__restrict__ x32, FwdOut o) {
   if (stopped(o.st)) return;
   Acc4 a;
   const int64_t nn = (int64_t)g.N * g.N;
-  // two adjacent threads per ray, each tracing one half (row_entries_part);
-  // the pair adds its halves by a shuffle, every lane runs every trip
-  const int part = threadIdx.x & 1;
-  const int64_t np = ((int64_t)gridDim.x * blockDim.x) >> 1;
-  const int64_t trips = (nrays + np - 1) / np;
-  for (int64_t t = 0, r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 1; t < trips; ++t, r += np) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nrays;
+       r += (int64_t)gridDim.x * blockDim.x) {
     double acc = 0.0;
-    if (r < nrays)
-      row_entries_part(g, r, excl, part, [&](int col, double v) {
-        if (col >= 0 && col < nn) acc = fma((double)(float)v, (double)x32[col], acc);
-      });
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    if (r < nrays && part == 0) resid_row<ME>(r, acc, o, a);
+    row_entries(g, r, excl, [&](int col, double v) {
+      if (col >= 0 && col < nn) acc = fma((double)(float)v, (double)x32[col], acc);
+    });
+    resid_row<ME>(r, acc, o, a);
   }
-  // warp sums (no block barrier: a warp whose rays are short leaves at once)
-  double r2 = warp_sum(a.r2), rmr = warp_sum(a.rmr), p2 = 0, pr = 0;
-  if (ME) {
-    p2 = warp_sum(a.p2);
-    pr = warp_sum(a.pr);
+  flush_warp<ME>(o.st, a);
+}
+
+// Row sums A*x of the listed slow rays, two threads per ray.
+__global__ void __launch_bounds__(64)
+    k_sirt_slow_rows(RayGeom g, int nslow, bool excl, const int *__restrict__ rays,
+                     const float *__restrict__ x32, double *__restrict__ y, const SirtState *st) {
+  if (stopped(st)) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 1;
+  double acc = 0.0;
+  if (e < nslow)
+    slow_cells(g, rays[e], excl, t & 1, [&](int cell, double v) { acc = fma(v, (double)x32[cell], acc); });
+  acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+  if (e < nslow && !(t & 1)) y[rays[e]] = acc;
+}
+
+// r = b - A*x over straight rays: warp w of a block walks part w of the
+// block's 32 rays (dda.cuh), gathering from the column- or row-major image;
+// the parts are added in order and warp 0 closes the rows.
+template <bool ME, bool UNIT>
+__global__ void __launch_bounds__(32 * kDdaParts, 4) k_sirt_fwd_dda(RayGeom g, int nrays, const float *__restrict__ x32,
+                               const float *__restrict__ x32t, const double *__restrict__ slow_y, FwdOut o) {
+  if (stopped(o.st)) return;
+  __shared__ double sh[kDdaParts][32];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5, parts = blockDim.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
+  // the products run two cells behind the gathers, which hides the gathers'
+  // latency without more warps
+  double acc = 0.0;
+  double v1 = 0.0, v2 = 0.0;
+  float x1 = 0.f, x2 = 0.f;
+  bool walked = true;
+  if (r < nrays)
+    walked = ray_cells<UNIT>(g, r, part, parts, [&](int cell, bool swapped, double v) {
+      acc = fma(v2, (double)x2, acc);
+      v2 = v1;
+      x2 = x1;
+      v1 = v;
+      x1 = __ldg((swapped ? x32t : x32) + cell);
+    });
+  acc = fma(v2, (double)x2, acc);
+  acc = fma(v1, (double)x1, acc);
+  sh[part][lane] = acc;
+  __syncthreads();
+  if (part != 0) return;
+  Acc4 a;
+  if (r < nrays) {
+    for (int q = 1; q < parts; ++q) acc += sh[q][lane];
+    if (!walked) acc = slow_y[r];
+    resid_row<ME>(r, acc, o, a);
   }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&o.st->acc[0], r2);
-    atomicAdd(&o.st->acc[1], rmr);
-    if (ME) {
-      atomicAdd(&o.st->acc[2], p2);
-      atomicAdd(&o.st->acc[3], pr);
-    }
-  }
+  flush_warp<ME>(o.st, a);
 }
 
 struct UpdArgs {
@@ -180,7 +230,19 @@ struct UpdArgs {
   const int *save_slot;
   SirtState *st;
   double *g64;
+  float *x32t;  // row-major FP32 copy of the N x N image (walks), or null
+  int N;
 };
+
+__device__ __forceinline__ void store_x(int64_t j, double x, const UpdArgs &u, int slot) {
+  u.x64[j] = x;
+  u.x32[j] = (float)x;
+  if (u.x32t) {
+    const int c = (int)j / u.N, r = (int)j - c * u.N;
+    u.x32t[(int64_t)r * u.N + c] = (float)x;
+  }
+  if (slot >= 0) u.X[(int64_t)slot * u.n + j] = x;
+}
 
 __device__ __forceinline__ void update_x(int64_t j, double g, double lam, const UpdArgs &u, int slot) {
   double x = u.x64[j] + lam * (u.D[j] * g);
@@ -188,9 +250,7 @@ __device__ __forceinline__ void update_x(int64_t j, double g, double lam, const 
   else if (u.lbk == AIRT_BOUND_VECTOR) x = fmax(x, u.lbv[j]);
   if (u.ubk == AIRT_BOUND_SCALAR) x = fmin(x, u.ub);
   else if (u.ubk == AIRT_BOUND_VECTOR) x = fmin(x, u.ubv[j]);
-  u.x64[j] = x;
-  u.x32[j] = (float)x;
-  if (slot >= 0) u.X[(int64_t)slot * u.n + j] = x;
+  store_x(j, x, u, slot);
 }
 
 // update_x with x64[j] and D[j] already loaded.
@@ -201,9 +261,7 @@ __device__ __forceinline__ void update_x_pre(int64_t j, double g, double lam, co
   else if (u.lbk == AIRT_BOUND_VECTOR) x = fmax(x, u.lbv[j]);
   if (u.ubk == AIRT_BOUND_SCALAR) x = fmin(x, u.ub);
   else if (u.ubk == AIRT_BOUND_VECTOR) x = fmin(x, u.ubv[j]);
-  u.x64[j] = x;
-  u.x32[j] = (float)x;
-  if (slot >= 0) u.X[(int64_t)slot * u.n + j] = x;
+  store_x(j, x, u, slot);
 }
 
 // MODE 0: fused update with st->lam_cur.  MODE 1: line-search pass that
@@ -258,6 +316,24 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamCtasPerSm)
     a4 = block_sum<kStreamThreads>(a4);
     if (threadIdx.x == 0) atomicAdd(&u.st->acc[4], a4);
   }
+}
+
+// Fused pixel-driven back projection and update (gather.cuh): warp w of a
+// block sums the angles w, w + warps, ... of the block's 32 pixels, warp 0
+// adds the sums in order and applies the update.
+__global__ void __launch_bounds__(32 * kGatherWarps, 5)
+    k_sirt_bwd_par(ParGather t, RayGeom g, const float *__restrict__ mr32, UpdArgs u) {
+  if (stopped(u.st)) return;
+  __shared__ double sh[kGatherWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  double acc = j < u.n ? par_sum(t, g, mr32, j, w, kGatherWarps) : 0.0;
+  sh[w][lane] = acc;
+  __syncthreads();
+  if (w != 0 || j >= u.n) return;
+  for (int q = 1; q < kGatherWarps; ++q) acc += sh[q][lane];
+  acc += par_fixes(t, mr32, j);
+  update_x(j, acc, u.st->lam_cur, u, u.save_slot[u.st->iter]);
 }
 
 // Elementwise update from a stored g (line search and matrix-free paths).
@@ -446,10 +522,16 @@ __global__ void k_sirt_ctrl(SirtState *st, const SirtParams *p) {
   }
 }
 
-__global__ void k_to_f32(int64_t n, const double *__restrict__ a, float *__restrict__ b) {
+__global__ void k_to_f32(int64_t n, const double *__restrict__ a, float *__restrict__ b,
+                         float *__restrict__ bt, int N) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
+       i += (int64_t)gridDim.x * blockDim.x) {
     b[i] = (float)a[i];
+    if (bt) {
+      const int c = (int)i / N, r = (int)i - c * N;
+      bt[(int64_t)r * N + c] = (float)a[i];
+    }
+  }
 }
 
 __global__ void k_copy(int64_t n, const double *__restrict__ a, double *__restrict__ b) {
@@ -498,9 +580,22 @@ void launch_fwd_t(Problem &P, const FwdOut &o) {
     return;
   }
   if (P.matrix_free) {
-    k_sirt_fwd_mf<ME><<<grid_for(2 * P.m, 64, 32), 64, 0, s>>>(P.geom(), P.m,
-                                                              P.geo_kind == GEO_PARALLEL,
-                                                              P.x32.p, o);
+    const bool excl = P.geo_kind == GEO_PARALLEL;
+    const unsigned gd = (unsigned)((P.m + 31) / 32), td = 32u * dda_parts(P.m);
+    if (P.m == 0) return;
+    if (P.geo_kind == GEO_SPHERE) {
+      k_sirt_fwd_mf<ME><<<grid_for(P.m, 64, 32), 64, 0, s>>>(P.geom(), P.m, excl, P.x32.p, o);
+      return;
+    }
+    if (P.nslow) {
+      P.slow_y.ensure(P.m);
+      k_sirt_slow_rows<<<(unsigned)((2 * (int64_t)P.nslow + 63) / 64), 64, 0, s>>>(
+          P.geom(), P.nslow, excl, P.slow_rays.p, P.x32.p, P.slow_y.p, o.st);
+    }
+    if (P.geo_kind == GEO_SEISMIC)
+      k_sirt_fwd_dda<ME, false><<<gd, td, 0, s>>>(P.geom(), (int)P.m, P.x32.p, P.x32t.p, P.slow_y.p, o);
+    else
+      k_sirt_fwd_dda<ME, true><<<gd, td, 0, s>>>(P.geom(), (int)P.m, P.x32.p, P.x32t.p, P.slow_y.p, o);
     return;
   }
   const int L = vec_lanes_for(P.nnz, P.m);
@@ -556,6 +651,9 @@ void launch_bwd(Problem &P, const UpdArgs &u, int relax_kind, const double *Dful
     }
     if (line) k_dense_D_update<true><<<dense_grid(P.n), 256, 0, s>>>(Dfull, P.g64.p, u);
     else k_dense_D_update<false><<<dense_grid(P.n), 256, 0, s>>>(Dfull, P.g64.p, u);
+  } else if (P.matrix_free && P.par_ok && !line) {
+    k_sirt_bwd_par<<<(unsigned)((P.n + 31) / 32), 32 * kGatherWarps, 0, s>>>(par_gather_of(P), P.geom(),
+                                                                            P.mr32.p, u);
   } else if (P.matrix_free) {
     mf_backproject_f32(P, P.mr32.p, P.g64.p, &P.state.p->stop);
     if (relax_kind == AIRT_RELAX_LINE) {
@@ -665,7 +763,9 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
     k_copy<<<grid_for(n, kThreads), kThreads, 0, s>>>(n, d_x0, P.x64.p);
   else
     AIRT_CHECK_CUDA(cudaMemsetAsync(P.x64.p, 0, n * sizeof(double), s));
-  k_to_f32<<<grid_for(n, kThreads), kThreads, 0, s>>>(n, P.x64.p, P.x32.p);
+  const bool walks = P.matrix_free && P.geo_kind != GEO_SPHERE;
+  if (walks) P.x32t.ensure(n);
+  k_to_f32<<<grid_for(n, kThreads), kThreads, 0, s>>>(n, P.x64.p, P.x32.p, walks ? P.x32t.p : nullptr, P.N);
   AIRT_LAUNCH_CHECK();
   if (me) AIRT_CHECK_CUDA(cudaMemsetAsync(P.rprev.p, 0, m * sizeof(double), s));
   if (o.lb_kind == AIRT_BOUND_VECTOR) {
@@ -733,6 +833,8 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
   ua.save_slot = P.save_slot.p;
   ua.st = P.state.p;
   ua.g64 = P.g64.p;
+  ua.x32t = walks ? P.x32t.p : nullptr;
+  ua.N = P.N;
 
   // forward pass, and with NCP the periodogram of the new residual
   const double *Dfull = dfull ? P.Dfull.p : nullptr;

@@ -17,12 +17,17 @@
 #include <climits>
 #include <cstring>
 
+#include <vector>
+
 #include "common.cuh"
+#include "gather.cuh"
 #include "spmv.cuh"
 #include "stream.cuh"
 #include "trace.cuh"
 
 namespace airt {
+
+ParGather par_gather_of(const Problem &P);
 
 namespace {
 
@@ -103,6 +108,7 @@ __global__ void k_absmax(int64_t n, const double *__restrict__ u, const float *_
     atomicMax(bits, (unsigned long long)__double_as_longlong(m));
 }
 
+// The terms of sphericaltomo's circles (one thread per circle).
 template <typename TU>
 __global__ void k_mf_adjoint_fx(RayGeom g, int64_t nrays, bool excl, const TU *__restrict__ u,
                                 long long *__restrict__ acc, double kbound,
@@ -113,21 +119,211 @@ __global__ void k_mf_adjoint_fx(RayGeom g, int64_t nrays, bool excl, const TU *_
   if (e == INT_MIN || e == INT_MAX) return;  // u == 0 (result 0) or not finite (NaN)
   const double sc = ldexp(1.0, 62 - e);
   const int64_t nn = (int64_t)g.N * g.N;
-  // two adjacent threads per ray, each scattering one half of its entries
-  // (row_entries_part): the entries are the same, and integer sums do not
-  // depend on their order
-  const int part = threadIdx.x & 1;
-  for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 1; r < nrays;
-       r += ((int64_t)gridDim.x * blockDim.x) >> 1) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nrays;
+       r += (int64_t)gridDim.x * blockDim.x) {
     const double ur = (double)u[r];
     if (ur == 0.0) continue;
-    row_entries_part(g, r, excl, part, [&](int col, double v) {
+    row_entries(g, r, excl, [&](int col, double v) {
       if (col >= 0 && col < nn) {
         const long long t = __double2ll_rn(__dmul_rn((double)(float)v, ur) * sc);
         atomicAdd(reinterpret_cast<unsigned long long *>(acc + col), (unsigned long long)t);
       }
     });
   }
+}
+
+// The terms of straight rays: warp w of a block walks part w of the block's
+// 32 rays (dda.cuh), so that the lanes of a warp scatter to neighbouring
+// pixels; walks along y go to the row-major sums acct.  u null: all ones.
+template <bool UNIT, typename TU>
+__global__ void __launch_bounds__(32 * kDdaParts, 4) k_dda_adjoint_fx(RayGeom g, int nrays, const TU *__restrict__ u,
+                                 unsigned long long *__restrict__ acc,
+                                 unsigned long long *__restrict__ acct, double kbound,
+                                 const unsigned long long *__restrict__ umax_bits, const int *stop_flag) {
+  if (stop_flag && *(volatile const int *)stop_flag) return;
+  const int e = fx_exponent(kbound, umax_bits ? __longlong_as_double((long long)*umax_bits) : 1.0);
+  if (e == INT_MIN || e == INT_MAX) return;  // u == 0 (result 0) or not finite (NaN)
+  const int r = blockIdx.x * 32 + (threadIdx.x & 31);
+  if (r >= nrays) return;
+  const double us = (u ? (double)u[r] : 1.0) * ldexp(1.0, 62 - e);  // exact scaling
+  if (us == 0.0) return;
+  ray_cells<UNIT>(g, r, threadIdx.x >> 5, blockDim.x >> 5, [&](int cell, bool swapped, double v) {
+    const long long t = __double2ll_rn(__dmul_rn(v, us));
+    atomicAdd((swapped ? acct : acc) + cell, (unsigned long long)t);
+  });
+}
+
+// The terms of the listed slow rays, two threads per ray.
+template <typename TU>
+__global__ void __launch_bounds__(64)
+    k_slow_adjoint_fx(RayGeom g, int nslow, bool excl, const int *__restrict__ rays, const TU *__restrict__ u,
+                      unsigned long long *__restrict__ acc, double kbound,
+                      const unsigned long long *__restrict__ umax_bits, const int *stop_flag) {
+  if (stop_flag && *(volatile const int *)stop_flag) return;
+  const int e = fx_exponent(kbound, umax_bits ? __longlong_as_double((long long)*umax_bits) : 1.0);
+  if (e == INT_MIN || e == INT_MAX) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >> 1 >= nslow) return;
+  const int r = rays[t >> 1];
+  const double us = (u ? (double)u[r] : 1.0) * ldexp(1.0, 62 - e);
+  if (us == 0.0) return;
+  slow_cells(g, r, excl, t & 1, [&](int cell, double v) {
+    atomicAdd(acc + cell, (unsigned long long)__double2ll_rn(__dmul_rn(v, us)));
+  });
+}
+
+// out = acc + transpose(acct) as integers, then FP64 (out and acc are the
+// same array).
+__global__ void k_fx_merge_f64(int N, double *__restrict__ out, const long long *__restrict__ acct,
+                               double kbound, const unsigned long long *__restrict__ umax_bits,
+                               const int *stop_flag) {
+  if (stop_flag && *(volatile const int *)stop_flag) return;
+  __shared__ long long t[32][33];
+  const int e = fx_exponent(kbound, umax_bits ? __longlong_as_double((long long)*umax_bits) : 1.0);
+  const double inv = e == INT_MIN ? 0.0 : e == INT_MAX ? __longlong_as_double(0x7ff8000000000000LL)
+                                                       : ldexp(1.0, e - 62);
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;  // columns (x) and rows of the tile
+  for (int q = threadIdx.y; q < 32; q += blockDim.y)
+    if (r0 + q < N && c0 + threadIdx.x < N) t[q][threadIdx.x] = acct[(int64_t)(r0 + q) * N + c0 + threadIdx.x];
+  __syncthreads();
+  long long *acc = reinterpret_cast<long long *>(out);
+  for (int q = threadIdx.y; q < 32; q += blockDim.y)
+    if (c0 + q < N && r0 + threadIdx.x < N) {
+      const int64_t j = (int64_t)(c0 + q) * N + r0 + threadIdx.x;
+      out[j] = (double)(acc[j] + t[threadIdx.x][q]) * inv;
+    }
+}
+
+// dst = transpose(src), N x N.
+template <typename T>
+__global__ void k_transpose_img(int N, const T *__restrict__ src, T *__restrict__ dst) {
+  __shared__ T t[32][33];
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  for (int q = threadIdx.y; q < 32; q += blockDim.y)
+    if (c0 + q < N && r0 + threadIdx.x < N) t[q][threadIdx.x] = src[(int64_t)(c0 + q) * N + r0 + threadIdx.x];
+  __syncthreads();
+  for (int q = threadIdx.y; q < 32; q += blockDim.y)
+    if (r0 + q < N && c0 + threadIdx.x < N) dst[(int64_t)(r0 + q) * N + c0 + threadIdx.x] = t[threadIdx.x][q];
+}
+
+// y = A*x over straight rays: the parts of a ray are added in order.
+template <bool UNIT>
+__global__ void k_dda_forward(RayGeom g, int nrays, const double *__restrict__ x,
+                              const double *__restrict__ xt, double *__restrict__ y) {
+  __shared__ double sh[kDdaParts][32];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5, parts = blockDim.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
+  double acc = 0.0;
+  bool walked = false;
+  if (r < nrays)
+    walked = ray_cells<UNIT>(g, r, part, parts, [&](int cell, bool swapped, double v) {
+      acc = fma(v, __ldg((swapped ? xt : x) + cell), acc);
+    });
+  sh[part][lane] = acc;
+  __syncthreads();
+  if (part == 0 && walked) {
+    for (int q = 1; q < parts; ++q) acc += sh[q][lane];
+    y[r] = acc;
+  }
+}
+
+// The listed slow rays' rows of y = A*x (x given) or of s2 and s1 (two
+// threads per ray).
+__global__ void __launch_bounds__(64)
+    k_slow_rows(RayGeom g, int nslow, bool excl, const int *__restrict__ rays, const double *__restrict__ x,
+                double *__restrict__ y, double *__restrict__ s2, double *__restrict__ s1) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 1;
+  double a = 0.0, a2 = 0.0, a1 = 0.0;
+  if (e < nslow)
+    slow_cells(g, rays[e], excl, t & 1, [&](int cell, double v) {
+      if (x) a = fma(v, x[cell], a);
+      a2 = fma(v, v, a2);
+      a1 += v;
+    });
+  a += __shfl_xor_sync(0xffffffffu, a, 1);
+  a2 += __shfl_xor_sync(0xffffffffu, a2, 1);
+  a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
+  if (e >= nslow || (t & 1)) return;
+  if (y) y[rays[e]] = a;
+  if (s2) s2[rays[e]] = a2;
+  if (s1) s1[rays[e]] = a1;
+}
+
+// Lists the slow rays and counts them in *cnt (at most m).
+__global__ void k_list_slow(RayGeom g, int nrays, int *__restrict__ list, int *__restrict__ cnt) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < nrays && dda_slow(g.N, ray_of(g, r))) list[atomicAdd(cnt, 1)] = r;
+}
+
+// Row sums of v^2 and |v| over straight rays.
+template <bool UNIT>
+__global__ void k_dda_row_stats(RayGeom g, int nrays, double *__restrict__ s2,
+                                double *__restrict__ s1) {
+  __shared__ double sh2[kDdaParts][32], sh1[kDdaParts][32];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5, parts = blockDim.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
+  double a2 = 0.0, a1 = 0.0;
+  bool walked = false;
+  if (r < nrays)
+    walked = ray_cells<UNIT>(g, r, part, parts, [&](int, bool, double v) {
+      a2 = fma(v, v, a2);
+      a1 += v;
+    });
+  sh2[part][lane] = a2;
+  sh1[part][lane] = a1;
+  __syncthreads();
+  if (part == 0 && walked) {
+    for (int q = 1; q < parts; ++q) {
+      a2 += sh2[q][lane];
+      a1 += sh1[q][lane];
+    }
+    if (s2) s2[r] = a2;
+    if (s1) s1[r] = a1;
+  }
+}
+
+// Pixel-driven back projection: warp w of a block sums the angles w, w +
+// warps, ... of the block's 32 pixels; the warps' sums are added in order.
+template <typename TU>
+__global__ void __launch_bounds__(32 * kGatherWarps, 5)
+    k_par_gather(ParGather t, RayGeom g, int n, const TU *__restrict__ u, double *__restrict__ out,
+                 const int *stop_flag) {
+  if (stop_flag && *(volatile const int *)stop_flag) return;
+  __shared__ double sh[kGatherWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  double acc = j < n ? par_sum(t, g, u, j, w, kGatherWarps) : 0.0;
+  sh[w][lane] = acc;
+  __syncthreads();
+  if (w == 0 && j < n) {
+    for (int q = 1; q < kGatherWarps; ++q) acc += sh[q][lane];
+    out[j] = acc + par_fixes(t, u, j);
+  }
+}
+
+// The corrections of the rays through the image's corners: for each listed
+// ray and each of its pixels, the traced entry less the closed form's (which
+// gives a pixel the reference dropped, too).  cand: the corner pixels.
+__global__ void k_par_fixes(ParGather t, RayGeom g, int nslow, const int *__restrict__ rays,
+                            ParFix *__restrict__ fix, int *__restrict__ cnt) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= 4 * nslow) return;
+  const int r = rays[q >> 2], c = q & 3, N = t.N;
+  const int ix = c & 1 ? N - 1 : 0, iy = c & 2 ? N - 1 : 0;
+  if (N == 1 && c) return;
+  const int j = ix * N + (N - 1 - iy), a = r / t.p, k = r - a * t.p;
+  const ParAngle A = t.ang[a];
+  if (!(A.ipq > 0.0)) return;
+  double v = 0.0;
+  trace_entries(N, ray_of(g, r), true, [&](int col, double len) {
+    if (col == j) v += (double)(float)len;
+  });
+  const double h = 0.5 * (double)N;
+  const double d = fma((double)k, t.D, t.s0) - fma(A.s, (double)iy + 0.5 - h, A.c * ((double)ix + 0.5 - h));
+  const double f = par_chord(A.w, A.ip, A.ipq, d);
+  if (v == f) return;
+  const int e = atomicAdd(cnt, 1);
+  if (e < kParFixMax) fix[e] = ParFix{j, r, v - f};
 }
 
 // Fixed-point sums back to FP64, in place (acc and out are the same array).
@@ -144,7 +340,7 @@ __global__ void k_fx_to_f64(int64_t n, double *__restrict__ out, double kbound,
 }
 
 // Terms each pixel receives and the largest entry, over every ray (the
-// bounds of the fixed-point scale).
+// bounds of the fixed-point scale); counts as the sums are scattered.
 __global__ void k_mf_emit_stats(RayGeom g, int64_t nrays, bool excl, int *__restrict__ cnt,
                                 unsigned long long *__restrict__ vmax_bits) {
   const int64_t nn = (int64_t)g.N * g.N;
@@ -158,6 +354,34 @@ __global__ void k_mf_emit_stats(RayGeom g, int64_t nrays, bool excl, int *__rest
       }
     });
   if (vm > 0.0) atomicMax(vmax_bits, (unsigned long long)__double_as_longlong(vm));
+}
+
+__global__ void __launch_bounds__(64)
+    k_slow_emit_stats(RayGeom g, int nslow, bool excl, const int *__restrict__ rays, int *__restrict__ cnt,
+                      unsigned long long *__restrict__ vmax_bits) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >> 1 >= nslow) return;
+  double vm = 0.0;
+  slow_cells(g, rays[t >> 1], excl, t & 1, [&](int cell, double v) {
+    atomicAdd(cnt + cell, 1);
+    vm = fmax(vm, v);
+  });
+  if (vm > 0.0) atomicMax(vmax_bits, (unsigned long long)__double_as_longlong(vm));
+}
+
+template <bool UNIT>
+__global__ void k_dda_emit_stats(RayGeom g, int nrays, int *__restrict__ cnt,
+                                 int *__restrict__ cntt, unsigned long long *__restrict__ vmax_bits) {
+  const int r = blockIdx.x * 32 + (threadIdx.x & 31);
+  double vm = 0.0;
+  if (r < nrays)
+    ray_cells<UNIT>(g, r, threadIdx.x >> 5, blockDim.x >> 5, [&](int cell, bool swapped, double v) {
+      atomicAdd((swapped ? cntt : cnt) + cell, 1);
+      vm = fmax(vm, v);
+    });
+  for (int o = 16; o > 0; o >>= 1) vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, o));
+  if ((threadIdx.x & 31) == 0 && vm > 0.0)
+    atomicMax(vmax_bits, (unsigned long long)__double_as_longlong(vm));
 }
 
 __global__ void k_max_int(int64_t n, const int *__restrict__ a, int *__restrict__ out) {
@@ -201,6 +425,96 @@ __global__ void k_mf_stats(RayGeom g, int64_t nrays, bool excl, double *__restri
 }
 
 inline bool excl_of(const Problem &P) { return P.geo_kind == GEO_PARALLEL; }
+inline unsigned slow_grid(const Problem &P) { return (unsigned)((2 * (int64_t)P.nslow + 63) / 64); }
+inline bool straight(const Problem &P) { return P.geo_kind != GEO_SPHERE; }
+
+// Launches KERNEL<UNIT> over the rays, dda_parts(m) warps of 32 rays per block.
+#define AIRT_DDA_LAUNCH(KERNEL, ...)                                                           \
+  do {                                                                                        \
+    const unsigned g_ = (unsigned)((P.m + 31) / 32), t_ = 32u * dda_parts(P.m);                 \
+    if (P.geo_kind == GEO_SEISMIC) KERNEL<false><<<g_, t_, 0, s>>>(P.geom(), (int)P.m, __VA_ARGS__); \
+    else KERNEL<true><<<g_, t_, 0, s>>>(P.geom(), (int)P.m, __VA_ARGS__);                        \
+  } while (0)
+
+template <typename TU>
+void dda_adjoint(Problem &P, const TU *u, double *out, const unsigned long long *umax, const int *stop) {
+  cudaStream_t s = P.stream;
+  const unsigned g_ = (unsigned)((P.m + 31) / 32), t_ = 32u * dda_parts(P.m);
+  unsigned long long *acc = reinterpret_cast<unsigned long long *>(out);
+  P.fxt.ensure(P.n);
+  unsigned long long *acct = reinterpret_cast<unsigned long long *>(P.fxt.p);
+  AIRT_CHECK_CUDA(cudaMemsetAsync(acc, 0, P.n * sizeof(double), s));
+  AIRT_CHECK_CUDA(cudaMemsetAsync(acct, 0, P.n * sizeof(double), s));
+  if (P.m) {
+    if (P.geo_kind == GEO_SEISMIC)
+      k_dda_adjoint_fx<false, TU><<<g_, t_, 0, s>>>(P.geom(), (int)P.m, u, acc, acct, P.mf_kbound, umax, stop);
+    else
+      k_dda_adjoint_fx<true, TU><<<g_, t_, 0, s>>>(P.geom(), (int)P.m, u, acc, acct, P.mf_kbound, umax, stop);
+    if (P.nslow)
+      k_slow_adjoint_fx<TU><<<slow_grid(P), 64, 0, s>>>(P.geom(), P.nslow, excl_of(P), P.slow_rays.p, u, acc,
+                                                        P.mf_kbound, umax, stop);
+  }
+  const unsigned tn = (unsigned)((P.N + 31) / 32);
+  k_fx_merge_f64<<<dim3(tn, tn), dim3(32, 8), 0, s>>>(P.N, out, P.fxt.p, P.mf_kbound, umax, stop);
+  AIRT_LAUNCH_CHECK();
+}
+
+template <typename TU>
+void par_backproject(Problem &P, const TU *u, double *out, const int *stop) {
+  k_par_gather<TU><<<(unsigned)((P.n + 31) / 32), 32 * kGatherWarps, 0, P.stream>>>(
+      par_gather_of(P), P.geom(), (int)P.n, u, out, stop);
+  AIRT_LAUNCH_CHECK();
+}
+
+// The angle records of the pixel-driven back projection, when the geometry
+// takes it: parallel rays at uniform offsets (to a few ulps), every angle
+// axis-parallel or inclined by at least kDdaSlope.
+void par_prepare(Problem &P) {
+  P.par_ok = false;
+  if (P.geo_kind != GEO_PARALLEL || P.p < 2 || P.nA < 1 || P.n >= INT_MAX - 32) return;
+  cudaStream_t s = P.stream;
+  std::vector<double> off(P.p), c(P.nA), sn(P.nA);
+  AIRT_CHECK_CUDA(cudaMemcpyAsync(off.data(), P.offsets.p, P.p * sizeof(double), cudaMemcpyDeviceToHost, s));
+  AIRT_CHECK_CUDA(cudaMemcpyAsync(c.data(), P.cos_t.p, P.nA * sizeof(double), cudaMemcpyDeviceToHost, s));
+  AIRT_CHECK_CUDA(cudaMemcpyAsync(sn.data(), P.sin_t.p, P.nA * sizeof(double), cudaMemcpyDeviceToHost, s));
+  AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+  const double D = (off[P.p - 1] - off[0]) / (P.p - 1);
+  // far finer rays than pixels would make a pixel's inner loop long
+  if (!(D > 1.0 / 64) || !std::isfinite(D)) return;
+  const double tol = 8 * 2.2e-16 * std::fmax(std::fabs(off[0]), std::fabs(off[P.p - 1]));
+  for (int k = 0; k < P.p; ++k)
+    if (!(std::fabs(off[k] - (off[0] + k * D)) <= tol)) return;
+  std::vector<ParAngle> t(P.nA);
+  for (int i = 0; i < P.nA; ++i) {
+    const double fc = std::fabs(c[i]), fs = std::fabs(sn[i]);
+    const double p = std::fmax(fc, fs), q = std::fmin(fc, fs);
+    if (!(std::fabs(p * p + q * q - 1.0) < 1e-14) || (q != 0.0 && q < kDdaSlope)) return;
+    t[i] = ParAngle{c[i], sn[i], 0.5 * (p + q), 1.0 / p, q != 0.0 ? 1.0 / (p * q) : 0.0,
+                    (-0.5 * (p + q) - off[0]) / D};
+  }
+  static_assert(sizeof(ParAngle) == 6 * sizeof(double), "angle record");
+  P.par_ang.upload(reinterpret_cast<const double *>(t.data()), t.size() * 6, s);
+  AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+  P.par_s0 = off[0];
+  P.par_D = D;
+  P.par_nfix = 0;
+  if (P.nslow) {  // rays through the corners; a longer list leaves the scatter in place
+    DevBuf<int> cnt;
+    cnt.ensure(1);
+    static_assert(sizeof(ParFix) == 2 * sizeof(double), "correction record");
+    P.par_fix.ensure(2 * kParFixMax);
+    AIRT_CHECK_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int), s));
+    k_par_fixes<<<(unsigned)((4 * (int64_t)P.nslow + 63) / 64), 64, 0, s>>>(
+        par_gather_of(P), P.geom(), P.nslow, P.slow_rays.p, reinterpret_cast<ParFix *>(P.par_fix.p), cnt.p);
+    AIRT_LAUNCH_CHECK();
+    int h = 0;
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(&h, cnt.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+    if (h > kParFixMax) return;
+    P.par_nfix = h;
+  }
+  P.par_ok = true;
+}
 
 }  // namespace
 
@@ -249,38 +563,78 @@ void mf_prepare(Problem &P) {
   AIRT_CHECK_CUDA(cudaMemsetAsync(cnt.p, 0, (P.n > 0 ? P.n : 1) * sizeof(int), s));
   AIRT_CHECK_CUDA(cudaMemsetAsync(cmax.p, 0, sizeof(int), s));
   AIRT_CHECK_CUDA(cudaMemsetAsync(vbits.p, 0, sizeof(unsigned long long), s));
-  if (P.m > 0)
+  DevBuf<int> cntt, cmaxt;  // walks along y count in the row-major image
+  cmaxt.ensure(1);
+  AIRT_CHECK_CUDA(cudaMemsetAsync(cmaxt.p, 0, sizeof(int), s));
+  if (P.m > 0 && straight(P)) {
+    cntt.ensure(P.n);
+    AIRT_CHECK_CUDA(cudaMemsetAsync(cntt.p, 0, P.n * sizeof(int), s));
+    P.slow_rays.ensure(P.m);
+    DevBuf<int> ns;
+    ns.ensure(1);
+    AIRT_CHECK_CUDA(cudaMemsetAsync(ns.p, 0, sizeof(int), s));
+    k_list_slow<<<(unsigned)((P.m + 255) / 256), 256, 0, s>>>(P.geom(), (int)P.m, P.slow_rays.p, ns.p);
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(&P.nslow, ns.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+    AIRT_DDA_LAUNCH(k_dda_emit_stats, cnt.p, cntt.p, vbits.p);
+    if (P.nslow)
+      k_slow_emit_stats<<<slow_grid(P), 64, 0, s>>>(P.geom(), P.nslow, excl_of(P), P.slow_rays.p, cnt.p, vbits.p);
+    k_max_int<<<grid_for(P.n, 256), 256, 0, s>>>(P.n, cntt.p, cmaxt.p);
+  } else if (P.m > 0) {
     k_mf_emit_stats<<<grid_for(P.m, 128, 16), 128, 0, s>>>(P.geom(), P.m, excl_of(P), cnt.p,
                                                             vbits.p);
+  }
   if (P.n > 0) k_max_int<<<grid_for(P.n, 256), 256, 0, s>>>(P.n, cnt.p, cmax.p);
   AIRT_LAUNCH_CHECK();
-  int hmax = 0;
+  int hmax = 0, hmaxt = 0;
+  AIRT_CHECK_CUDA(cudaMemcpyAsync(&hmaxt, cmaxt.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   unsigned long long hv = 0;
   AIRT_CHECK_CUDA(cudaMemcpyAsync(&hmax, cmax.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   AIRT_CHECK_CUDA(cudaMemcpyAsync(&hv, vbits.p, sizeof(hv), cudaMemcpyDeviceToHost, s));
   AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
-  double T = 1.0;
-  while (T < (double)hmax) T *= 2.0;
+  double T = 1.0;  // a bound on a pixel's terms from both walks
+  while (T < (double)hmax + (double)hmaxt) T *= 2.0;
   double vmax = 0.0;
   std::memcpy(&vmax, &hv, sizeof(vmax));
   P.mf_kbound = T * (vmax > 0.0 ? vmax : 1.0);
   P.mf_umax.ensure(1);
+  par_prepare(P);
+}
+
+ParGather par_gather_of(const Problem &P) {
+  return ParGather{reinterpret_cast<const ParAngle *>(P.par_ang.p), P.par_s0, P.par_D, 1.0 / P.par_D, P.N, P.nA,
+                   P.p, reinterpret_cast<const ParFix *>(P.par_fix.p), P.par_nfix};
 }
 
 void apply_matrix_free(Problem &P, const double *d_in, double *d_out, int transp) {
   cudaStream_t s = P.stream;
   const RayGeom g = P.geom();
-  const unsigned grid = grid_for(P.m, 128, 16);
   if (!transp) {
-    k_mf_forward<<<grid, 128, 0, s>>>(g, P.m, excl_of(P), d_in, d_out);
+    if (P.m == 0) return;
+    if (straight(P)) {
+      P.x64t.ensure(P.n);
+      const unsigned tn = (unsigned)((P.N + 31) / 32);
+      k_transpose_img<double><<<dim3(tn, tn), dim3(32, 8), 0, s>>>(P.N, d_in, P.x64t.p);
+      AIRT_DDA_LAUNCH(k_dda_forward, d_in, P.x64t.p, d_out);
+      if (P.nslow)
+        k_slow_rows<<<slow_grid(P), 64, 0, s>>>(g, P.nslow, excl_of(P), P.slow_rays.p, d_in, d_out, nullptr,
+                                                nullptr);
+    } else {
+      k_mf_forward<<<grid_for(P.m, 128, 16), 128, 0, s>>>(g, P.m, excl_of(P), d_in, d_out);
+    }
+  } else if (P.par_ok) {
+    par_backproject<double>(P, d_in, d_out, nullptr);
   } else {
-    AIRT_CHECK_CUDA(cudaMemsetAsync(d_out, 0, P.n * sizeof(double), s));
     AIRT_CHECK_CUDA(cudaMemsetAsync(P.mf_umax.p, 0, sizeof(unsigned long long), s));
     k_absmax<<<grid_for(P.m, 256), 256, 0, s>>>(P.m, d_in, nullptr, P.mf_umax.p, nullptr);
-    k_mf_adjoint_fx<double><<<grid_for(2 * P.m, 128, 16), 128, 0, s>>>(g, P.m, excl_of(P), d_in,
-                                                 reinterpret_cast<long long *>(d_out),
-                                                 P.mf_kbound, P.mf_umax.p, nullptr);
-    k_fx_to_f64<<<grid_for(P.n, 256), 256, 0, s>>>(P.n, d_out, P.mf_kbound, P.mf_umax.p, nullptr);
+    if (straight(P)) {
+      dda_adjoint<double>(P, d_in, d_out, P.mf_umax.p, nullptr);
+    } else {
+      AIRT_CHECK_CUDA(cudaMemsetAsync(d_out, 0, P.n * sizeof(double), s));
+      k_mf_adjoint_fx<double><<<grid_for(P.m, 128, 16), 128, 0, s>>>(
+          g, P.m, excl_of(P), d_in, reinterpret_cast<long long *>(d_out), P.mf_kbound, P.mf_umax.p, nullptr);
+      k_fx_to_f64<<<grid_for(P.n, 256), 256, 0, s>>>(P.n, d_out, P.mf_kbound, P.mf_umax.p, nullptr);
+    }
   }
   AIRT_LAUNCH_CHECK();
 }
@@ -292,6 +646,20 @@ void row_col_stats_mf(Problem &P, double *s2, double *s1, double *colcnt, double
     return;
   }
   cudaStream_t s = P.stream;
+  // The counts of nonzeros need the traced entries (slivers count); sums do
+  // not.
+  if (!colcnt && !s2w) {
+    if ((s2 || s1) && P.m) {
+      AIRT_DDA_LAUNCH(k_dda_row_stats, s2, s1);
+      if (P.nslow)
+        k_slow_rows<<<slow_grid(P), 64, 0, s>>>(P.geom(), P.nslow, excl_of(P), P.slow_rays.p, nullptr, nullptr,
+                                                s2, s1);
+    }
+    if (cols1 && P.par_ok) par_backproject<double>(P, nullptr, cols1, nullptr);
+    else if (cols1) dda_adjoint<double>(P, nullptr, cols1, nullptr, nullptr);
+    AIRT_LAUNCH_CHECK();
+    return;
+  }
   if (colcnt) AIRT_CHECK_CUDA(cudaMemsetAsync(colcnt, 0, P.n * sizeof(double), s));
   if (cols1) AIRT_CHECK_CUDA(cudaMemsetAsync(cols1, 0, P.n * sizeof(double), s));
   k_mf_stats<<<grid_for(P.m, 128, 16), 128, 0, s>>>(P.geom(), P.m, excl_of(P), s2, s1, colcnt,
@@ -349,10 +717,18 @@ int64_t test_split_trace(Problem &P, int64_t *nsplit) {
 // Matrix-free pieces of the SIRT iteration (used by sirt.cu).
 void mf_backproject_f32(Problem &P, const float *u, double *g64, const int *stop_flag) {
   cudaStream_t s = P.stream;
-  AIRT_CHECK_CUDA(cudaMemsetAsync(g64, 0, P.n * sizeof(double), s));
+  if (P.par_ok) {
+    par_backproject<float>(P, u, g64, stop_flag);
+    return;
+  }
   AIRT_CHECK_CUDA(cudaMemsetAsync(P.mf_umax.p, 0, sizeof(unsigned long long), s));
   k_absmax<<<grid_for(P.m, 256), 256, 0, s>>>(P.m, nullptr, u, P.mf_umax.p, stop_flag);
-  k_mf_adjoint_fx<float><<<grid_for(2 * P.m, 64, 32), 64, 0, s>>>(
+  if (straight(P)) {
+    dda_adjoint<float>(P, u, g64, P.mf_umax.p, stop_flag);
+    return;
+  }
+  AIRT_CHECK_CUDA(cudaMemsetAsync(g64, 0, P.n * sizeof(double), s));
+  k_mf_adjoint_fx<float><<<grid_for(P.m, 64, 32), 64, 0, s>>>(
       P.geom(), P.m, excl_of(P), u, reinterpret_cast<long long *>(g64), P.mf_kbound, P.mf_umax.p,
       stop_flag);
   k_fx_to_f64<<<grid_for(P.n, 256), 256, 0, s>>>(P.n, g64, P.mf_kbound, P.mf_umax.p, stop_flag);
