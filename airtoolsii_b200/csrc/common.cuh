@@ -169,6 +169,18 @@ struct ArtSchedule {
   DevBuf<int> steps, pos, pred_ptr, preds;
 };
 
+// Plan of the blocked CART sweep for a column order without repeats
+// (cart.cu): blocks of kCartCols consecutive columns of the order, the
+// entries of a block sorted by row, and the columns' inner products.
+struct CartPlan {
+  int64_t nblocks = 0;
+  uint64_t key = 0;  // hash of the column order it was built for (0: none)
+  DevBuf<int> cols;              // the order
+  DevBuf<int64_t> cbase;         // nblocks + 1 offsets into the chunks
+  DevBuf<uint2> ent;             // chunks of 32 sorted entries: row | column of the block << 27, value bits
+  DevBuf<double> gram;           // nblocks x 2*kCartCols x kCartCols
+};
+
 // ---------------------------------------------------------------- problem
 struct Problem {
   int64_t m = 0, n = 0, nnz = 0;
@@ -229,6 +241,7 @@ struct Problem {
   // Kaczmarz schedule of the last fixed row order (kept between calls: the
   // matrix never changes, so the same order gives the same schedule)
   ArtSchedule art_sched;
+  CartPlan cart_plan;  // likewise for the last column order
   // multi-right-hand-side SIRT (multirhs.cu): interleaved [row or pixel][instance]
   DevBuf<double> mr_b, mr_x64, mr_part, mr_resn, mr_taud, mr_lam;
   DevBuf<float> mr_x32, mr_r32;
