@@ -329,6 +329,7 @@ int airt_apply_device(airt_problem *h, const double *d_in, double *d_out, int tr
   AIRT_API_BEGIN
   AIRT_REQUIRE(h && d_in && d_out, "null pointer argument");
   Problem *P = reinterpret_cast<Problem *>(h);
+  if (!P->matrix_free) AIRT_CHECK_CUDA(cudaStreamSynchronize(P->stream));
   apply_operator(*P, d_in, d_out, transp);
   AIRT_API_END
 }
@@ -338,9 +339,7 @@ int airt_weights(airt_problem *h, int method, double *M, double *D) {
   AIRT_REQUIRE(h && M && D, "null pointer argument");
   AIRT_REQUIRE(method >= AIRT_LANDWEBER && method <= AIRT_SART, "SIRT method not defined.");
   Problem *P = reinterpret_cast<Problem *>(h);
-  P->M.ensure(P->m);
-  P->D.ensure(P->n);
-  compute_weights(*P, method, P->M.p, P->D.p);
+  use_weights(*P, method);
   AIRT_CHECK_CUDA(cudaMemcpyAsync(M, P->M.p, P->m * sizeof(double), cudaMemcpyDeviceToHost, P->stream));
   AIRT_CHECK_CUDA(cudaMemcpyAsync(D, P->D.p, P->n * sizeof(double), cudaMemcpyDeviceToHost, P->stream));
   AIRT_CHECK_CUDA(cudaStreamSynchronize(P->stream));
@@ -356,6 +355,7 @@ int airt_rho(airt_problem *h, int method, const double *Mcustom, const double *D
   P->M.ensure(P->m);
   P->D.ensure(P->n);
   if (method == AIRT_CUSTOM) {
+    P->wt_method = -1;
     std::vector<double> ones;
     if (Mcustom) P->M.upload(Mcustom, P->m, P->stream);
     else {
@@ -370,7 +370,7 @@ int airt_rho(airt_problem *h, int method, const double *Mcustom, const double *D
     AIRT_CHECK_CUDA(cudaStreamSynchronize(P->stream));
   } else {
     AIRT_REQUIRE(method >= AIRT_LANDWEBER && method <= AIRT_SART, "SIRT method not defined.");
-    compute_weights(*P, method, P->M.p, P->D.p);
+    use_weights(*P, method);
   }
   *rho = estimate_rho(*P, P->M.p, P->D.p, tol, maxit);
   AIRT_API_END
@@ -394,6 +394,7 @@ int airt_rho_custom(airt_problem *h, const double *M, int M_full, const double *
   AIRT_REQUIRE(maxit > 0 && tol >= 0, "invalid tolerance or iteration limit");
   Problem *P = reinterpret_cast<Problem *>(h);
   const bool mf = M && M_full, df = D && D_full;
+  P->wt_method = -1;
   AIRT_REQUIRE(!mf || (double)P->m * (double)P->m <= 4e9, "a full custom M does not fit the device");
   AIRT_REQUIRE(!df || (double)P->n * (double)P->n <= 4e9, "a full custom D does not fit the device");
   const double *dM = nullptr, *dD = nullptr;

@@ -136,6 +136,7 @@ struct SirtState {
   double lam_cur; // relaxpar applied in the iteration being computed
   double lam_last;
   double rmr_prev;  // r'*M*r of the previous residual (line search numerator)
+  unsigned done;    // blocks of the running forward pass that have added their sums
 };
 
 // State of the multi-right-hand-side SIRT (multirhs.cu).
@@ -210,6 +211,7 @@ struct Problem {
   int nrtiles = 0, nctiles = 0;
   DevBuf<int> err;  // device error flag (bounded waits)
 
+  int wt_method = -1;  // built-in method whose weights M and D hold (use_weights)
   // reusable scratch of the weight and rho computations
   DevBuf<double> w1, w2;
   // matrix-free back projection in fixed point (trace.cu): bound on
@@ -255,6 +257,8 @@ struct Problem {
   DevBuf<float> x32, mr32;
   DevBuf<SirtState> state;
   DevBuf<SirtParams> params;
+  DevBuf<double> pst_part;     // one-launch SIRT (persist.cuh): partial sums, barrier counter
+  DevBuf<unsigned> pst_count;
   DevBuf<int> save_slot;
   SirtState *h_state = nullptr;  // pinned mirror
 
@@ -333,6 +337,7 @@ void mf_prepare(Problem &P);
 int64_t test_split_trace(Problem &P, int64_t *nsplit);
 void apply_operator(Problem &P, const double *d_in, double *d_out, int transp);
 void compute_weights(Problem &P, int method, double *dM, double *dD);
+void use_weights(Problem &P, int method);
 void run_sirt_multi(Problem &P, const airt_sirt_opts &o, int K, const double *d_B,
                     const double *d_X0, const double *taud_host, const double *lam_host,
                     const int64_t *Ksave, int64_t nsave, double *d_Xs, double *d_X,

@@ -614,9 +614,7 @@ void run_sirt_multi(Problem &P, const airt_sirt_opts &o, int K, const double *d_
   AIRT_CHECK_CUDA(cudaEventCreate(&t0));
   AIRT_CHECK_CUDA(cudaEventCreate(&t1));
   AIRT_CHECK_CUDA(cudaEventRecord(t0, s));
-  P.M.ensure(P.m);
-  P.D.ensure(P.n);
-  compute_weights(P, o.method, P.M.p, P.D.p);
+  use_weights(P, o.method);
   const double *taud = o.stoprule == AIRT_STOP_DP ? taud_host : nullptr;
   for (int k0 = 0; k0 < K; k0 += kMaxK) {
     const int kc = std::min(kMaxK, K - k0);

@@ -10,13 +10,14 @@
 //   fwd : r = b - A*x over the CSR (gather of the FP32 copy of x), fused
 //         with M.*r (FP32 copy for the next gather) and the FP64 sums
 //         ||r||^2, r'*M*r and, for ME, the previous-residual products;
-//   ctrl: one thread applies the stopping rule to the sums, records
-//         ||r_k|| and the relaxpar used, and selects the next relaxpar.
+//   ctrl: the last block of the forward pass applies the stopping rule to the
+//         sums, records ||r_k|| and the relaxpar used, and selects the next.
 // Kernels read the device stop flag first and return at once after a stop,
 // so the host can enqueue iterations in chunks and poll the flag lazily.
 //
 // Precision: matrix values and the two gathered vectors are FP32; products
 // are accumulated in FP64; x, r, b, M, D and all reductions are FP64.
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -24,6 +25,7 @@
 #include "stream.cuh"
 #include "ncp.cuh"
 #include "gather.cuh"
+#include "persist.cuh"
 
 namespace airt {
 
@@ -34,12 +36,77 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// Stopping rule of check_stoprules.m on the sums of the residual just
+// computed, then the relaxpar of the next iteration (sirt.m:216-226).
+__device__ __forceinline__ void sirt_control(SirtState *st, const SirtParams *p) {
+  const int k = st->iter;
+  const double nrk = sqrt(st->acc[0]);
+  p->resn_hist[k] = nrk;
+  p->lam_hist[k] = st->lam_cur;
+  bool stop = false;
+  int rule = 0;
+  const int64_t kmax = p->kmax;
+  switch (p->stoprule) {
+    case AIRT_STOP_DP:  // check_stoprules.m:56-72
+      if (nrk <= p->taudelta || k >= kmax) {
+        stop = true;
+        rule = (k != kmax) ? 2 : 0;
+      }
+      break;
+    case AIRT_STOP_ME: {  // check_stoprules.m:74-94
+      const double np = sqrt(st->acc[2]);
+      const double dme = st->acc[3] / 2.0;
+      if (k > 0 && dme / np <= p->taudelta) {
+        stop = true;
+        rule = 3;
+      } else if (k >= kmax) {
+        stop = true;
+        rule = 0;
+      }
+      break;
+    }
+    case AIRT_STOP_NCP: {  // check_stoprules.m:97-150
+      double sum = 0.0;
+      for (int j = 0; j < p->ncp_cols; ++j) sum += p->ncc_col[j];
+      const double ncc = sum / p->ncp_cols;
+      const int ns = p->ncp_smooth;
+      double mx = -INFINITY, mxn = ncc;  // max(dk), max([dk(2:end); ncc]); NaN ignored
+      for (int i = 0; i < ns; ++i) mx = fmax(mx, p->dk[i]);
+      for (int i = 1; i < ns; ++i) mxn = fmax(mxn, p->dk[i]);
+      if (mx < mxn || k >= kmax) {
+        stop = true;
+        rule = (k != kmax) ? 1 : 0;
+      } else {
+        for (int i = 0; i + 1 < ns; ++i) p->dk[i] = p->dk[i + 1];
+        p->dk[ns - 1] = ncc;
+      }
+      break;
+    }
+    default:  // NONE, check_stoprules.m:153-161
+      if (k >= kmax) stop = true;
+  }
+  st->rmr_prev = st->acc[1];
+  for (int q = 0; q < 6; ++q) st->acc[q] = 0.0;
+  if (stop) {
+    st->stop = 1;
+    st->stoprule = rule;
+    st->finaliter = k;
+    st->lam_last = st->lam_cur;
+  } else {
+    const int kn = k + 1;
+    if (p->relax_kind == AIRT_RELAX_CONST) st->lam_cur = p->relaxpar;
+    else if (p->relax_kind == AIRT_RELAX_TABLE) st->lam_cur = p->relax_table[kn - 1];
+    st->iter = kn;
+  }
+}
+
 struct FwdOut {
   const double *b;
   const double *M;
   float *mr32;
   double *rprev;  // ME only
   SirtState *st;
+  const SirtParams *p;  // the last block to add its sums runs the control step; null: it does not
 };
 
 struct Acc4 {
@@ -77,8 +144,28 @@ __device__ __forceinline__ void resid_row(int64_t i, double s, const FwdOut &o, 
   }
 }
 
+// Adds one thread's sums to the state; the last of the grid's `adders` to
+// arrive runs the control step, which saves a launch per iteration (3 us).
 template <bool ME>
-__device__ __forceinline__ void flush(SirtState *st, Acc4 &a) {
+__device__ __forceinline__ void add_sums(const FwdOut &o, double r2, double rmr, double p2, double pr,
+                                         unsigned adders) {
+  SirtState *st = o.st;
+  atomicAdd(&st->acc[0], r2);
+  atomicAdd(&st->acc[1], rmr);
+  if (ME) {
+    atomicAdd(&st->acc[2], p2);
+    atomicAdd(&st->acc[3], pr);
+  }
+  if (!o.p) return;
+  __threadfence();
+  if (atomicAdd(&st->done, 1u) + 1u < adders) return;
+  __threadfence();
+  st->done = 0;
+  sirt_control(st, o.p);
+}
+
+template <bool ME>
+__device__ __forceinline__ void flush(const FwdOut &o, Acc4 &a) {
   double r2 = block_sum<kThreads>(a.r2);
   double rmr = block_sum<kThreads>(a.rmr);
   double p2 = 0, pr = 0;
@@ -86,33 +173,19 @@ __device__ __forceinline__ void flush(SirtState *st, Acc4 &a) {
     p2 = block_sum<kThreads>(a.p2);
     pr = block_sum<kThreads>(a.pr);
   }
-  if (threadIdx.x == 0) {
-    atomicAdd(&st->acc[0], r2);
-    atomicAdd(&st->acc[1], rmr);
-    if (ME) {
-      atomicAdd(&st->acc[2], p2);
-      atomicAdd(&st->acc[3], pr);
-    }
-  }
+  if (threadIdx.x == 0) add_sums<ME>(o, r2, rmr, p2, pr, gridDim.x);
 }
 
-// flush without a block barrier: one warp's sums.
+// flush without a block barrier: one warp's sums, of `warps` warps in all.
 template <bool ME>
-__device__ __forceinline__ void flush_warp(SirtState *st, Acc4 &a) {
+__device__ __forceinline__ void flush_warp(const FwdOut &o, Acc4 &a, unsigned warps) {
   const double r2 = warp_sum(a.r2), rmr = warp_sum(a.rmr);
   double p2 = 0, pr = 0;
   if (ME) {
     p2 = warp_sum(a.p2);
     pr = warp_sum(a.pr);
   }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&st->acc[0], r2);
-    atomicAdd(&st->acc[1], rmr);
-    if (ME) {
-      atomicAdd(&st->acc[2], p2);
-      atomicAdd(&st->acc[3], pr);
-    }
-  }
+  if ((threadIdx.x & 31) == 0) add_sums<ME>(o, r2, rmr, p2, pr, warps);
 }
 
 __device__ __forceinline__ bool stopped(const SirtState *st) {
@@ -133,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 4)
       [&](int64_t i, double s, bool lead, BM pv) {
         if (lead) resid_row_pre<ME>(i, s, o, a, pv.b, pv.m);
       });
-  flush<ME>(o.st, a);
+  flush<ME>(o, a);
 }
 
 // Streamed variants (stream.cuh): same epilogues, tiles of the CSR / CSC
@@ -146,7 +219,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamCtasPerSm)
   stream_segments(sa, [&](int64_t i, double s, bool lead) {
     if (lead) resid_row<ME>(i, s, o, a);
   });
-  flush<ME>(o.st, a);
+  flush<ME>(o, a);
 }
 
 // r = b - A*x over sphericaltomo's circles, one thread per circle.
@@ -164,7 +237,7 @@ __global__ void __launch_bounds__(64)
     });
     resid_row<ME>(r, acc, o, a);
   }
-  flush_warp<ME>(o.st, a);
+  flush_warp<ME>(o, a, gridDim.x * (blockDim.x >> 5));
 }
 
 // Row sums A*x of the listed slow rays, two threads per ray.
@@ -215,7 +288,7 @@ __global__ void __launch_bounds__(32 * kDdaParts, 4) k_sirt_fwd_dda(RayGeom g, i
     if (!walked) acc = slow_y[r];
     resid_row<ME>(r, acc, o, a);
   }
-  flush_warp<ME>(o.st, a);
+  flush_warp<ME>(o, a, gridDim.x);
 }
 
 struct UpdArgs {
@@ -253,8 +326,8 @@ __device__ __forceinline__ void update_x(int64_t j, double g, double lam, const 
   store_x(j, x, u, slot);
 }
 
-// update_x with x64[j] and D[j] already loaded.
-__device__ __forceinline__ void update_x_pre(int64_t j, double g, double lam, const UpdArgs &u, int slot,
+// update_x with x64[j] and D[j] already loaded; returns the new x(j).
+__device__ __forceinline__ double update_x_pre(int64_t j, double g, double lam, const UpdArgs &u, int slot,
                                              double x0, double dj) {
   double x = x0 + lam * (dj * g);
   if (u.lbk == AIRT_BOUND_SCALAR) x = fmax(x, u.lb);
@@ -262,6 +335,7 @@ __device__ __forceinline__ void update_x_pre(int64_t j, double g, double lam, co
   if (u.ubk == AIRT_BOUND_SCALAR) x = fmin(x, u.ub);
   else if (u.ubk == AIRT_BOUND_VECTOR) x = fmin(x, u.ubv[j]);
   store_x(j, x, u, slot);
+  return x;
 }
 
 // MODE 0: fused update with st->lam_cur.  MODE 1: line-search pass that
@@ -334,6 +408,113 @@ __global__ void __launch_bounds__(32 * kGatherWarps, 5)
   for (int q = 1; q < kGatherWarps; ++q) acc += sh[q][lane];
   acc += par_fixes(t, mr32, j);
   update_x(j, acc, u.st->lam_cur, u, u.save_slot[u.st->iter]);
+}
+
+// All iterations from it0 + 1 to it1 in one cooperative launch
+// (persist.cuh); it0 = 0 starts with the initial residual.  Rules NONE and DP,
+// constant or tabulated relaxpar.
+struct PersistArgs {
+  PersistDir rows, cols;
+  const double *b, *M;
+  float *mr32;
+  UpdArgs u;
+  const SirtParams *p;
+  double *part;      // 2 x grid partial sums of ||r||^2 (by parity of the iteration)
+  unsigned *count;   // barrier counter, zeroed before the launch
+  int *err;
+  long long budget;
+  int it0, it1;
+};
+
+template <int THREADS, int R>
+__global__ void __launch_bounds__(THREADS, 1) k_sirt_persist(const __grid_constant__ PersistArgs a) {
+  constexpr int kWarps = THREADS / 32, kAhead = R ? 1 : 2, kParts = 5;  // grids of up to 32 * kParts CTAs
+  __shared__ double nrk_sh, sums[kWarps];
+  const int gt = blockIdx.x * THREADS + threadIdx.x, total = gridDim.x * THREADS;
+  const int lr = gt % a.rows.L, lc = gt % a.cols.L;
+  const int gr = gt / a.rows.L, gc = gt / a.cols.L;        // first row / column of the group
+  const int nr = total / a.rows.L, nc = total / a.cols.L;  // groups
+  const PersistSeg<R> sr = persist_load<R>(a.rows, gr, lr), sc = persist_load<R>(a.cols, gc, lc);
+  const bool rown = lr == 0 && gr < a.rows.nseg, cown = lc == 0 && gc < a.cols.nseg;
+  const double b0 = rown ? a.b[gr] : 0.0, M0 = rown ? a.M[gr] : 0.0, D0 = cown ? a.u.D[gc] : 0.0;
+  double x0 = cown ? a.u.x64[gc] : 0.0;
+  unsigned target = 0;
+  auto first_dot = [&](const PersistDir &d, const PersistSeg<R> &seg, int i, int lane, const float *x) {
+    return persist_group_sum(R ? persist_dot(d, seg, x) : persist_dot_again<kAhead>(d, i, lane, x), d.L);
+  };
+  // r = b - A*x, M.*r and the warps' sums of ||r||^2; thread 0 adds them at
+  // the barrier that follows
+  auto forward = [&](int it) -> bool {
+    double s = first_dot(a.rows, sr, gr, lr, a.u.x32), r2 = 0.0;
+    if (rown) {
+      const double r = b0 - s;
+      a.mr32[gr] = (float)(M0 * r);
+      r2 = r * r;
+    }
+    for (int i = gr + nr; !__all_sync(0xffffffffu, i >= a.rows.nseg); i += nr) {
+      s = persist_group_sum(persist_dot_again<kAhead>(a.rows, i, lr, a.u.x32), a.rows.L);
+      if (lr == 0 && i < a.rows.nseg) {
+        const double r = a.b[i] - s;
+        a.mr32[i] = (float)(a.M[i] * r);
+        r2 += r * r;
+      }
+    }
+    r2 = warp_sum(r2);
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = r2;
+    return persist_barrier(a.count, target += gridDim.x, a.err, a.budget, [&] {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) v += sums[w];
+      a.part[(it & 1) * gridDim.x + blockIdx.x] = v;
+    });
+  };
+  if (a.it0 == 0 && !forward(0)) return;
+  const int kmax = (int)a.p->kmax, rule = a.p->stoprule;
+  const bool table = a.p->relax_kind == AIRT_RELAX_TABLE;
+  const double taud = a.p->taudelta, lam_const = a.p->relaxpar;
+  for (int it = a.it0 + 1;; ++it) {
+    // the update of iteration it, unless the residual of k = it - 1 stops the
+    // solve; warp 0 loads the CTAs' sums beside its gathers
+    const int k = it - 1;
+    double pv[kParts];
+#pragma unroll
+    for (int q = 0; q < kParts; ++q) {
+      const int c = threadIdx.x + 32 * q;
+      pv[q] = threadIdx.x < 32 && c < (int)gridDim.x ? a.part[(k & 1) * gridDim.x + c] : 0.0;
+    }
+    const double s = first_dot(a.cols, sc, gc, lc, a.mr32);
+    if (threadIdx.x < 32) {
+      double v = 0.0;
+#pragma unroll
+      for (int q = 0; q < kParts; ++q) v += pv[q];
+      v = warp_sum(v);
+      if (threadIdx.x == 0) nrk_sh = sqrt(v);
+    }
+    __syncthreads();
+    const double nrk = nrk_sh;
+    const bool stop = (rule == AIRT_STOP_DP && nrk <= taud) || k >= kmax;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (k > a.it0 || k == 0)) {
+      const double lam_k = k == 0 ? a.u.st->lam_cur : table ? a.p->relax_table[k - 1] : lam_const;
+      a.p->resn_hist[k] = nrk;
+      a.p->lam_hist[k] = lam_k;
+      if (stop) {
+        a.u.st->stop = 1;
+        a.u.st->stoprule = rule == AIRT_STOP_DP && k != kmax ? 2 : 0;
+        a.u.st->finaliter = k;
+        a.u.st->lam_last = lam_k;
+      }
+    }
+    if (stop || it > a.it1) return;
+    const int slot = a.u.save_slot[it];
+    const double lam = table ? a.p->relax_table[it - 1] : lam_const;
+    if (cown) x0 = update_x_pre(gc, s, lam, a.u, slot, x0, D0);
+    for (int j = gc + nc; !__all_sync(0xffffffffu, j >= a.cols.nseg); j += nc) {
+      const double g = persist_group_sum(persist_dot_again<kAhead>(a.cols, j, lc, a.mr32), a.cols.L);
+      if (lc == 0 && j < a.cols.nseg) update_x_pre(j, g, lam, a.u, slot, a.u.x64[j], a.u.D[j]);
+    }
+    if (!persist_barrier(a.count, target += gridDim.x, a.err, a.budget, [] {})) return;
+    if (!forward(it)) return;
+  }
 }
 
 // Elementwise update from a stored g (line search and matrix-free paths).
@@ -456,70 +637,12 @@ __global__ void k_colsum(int64_t k, const double *__restrict__ W, double *__rest
 
 inline unsigned dense_grid(int64_t k) { return (unsigned)((k + kGemvRows - 1) / kGemvRows); }
 
-// Stopping rule of check_stoprules.m on the sums of the residual just
-// computed, then the relaxpar of the next iteration (sirt.m:216-226).
+// The control step on its own, where kernels follow the forward pass before
+// its sums are complete (NCP, full custom M).
 __global__ void k_sirt_ctrl(SirtState *st, const SirtParams *p) {
   if (threadIdx.x || blockIdx.x) return;
   if (st->stop) return;
-  const int k = st->iter;
-  const double nrk = sqrt(st->acc[0]);
-  p->resn_hist[k] = nrk;
-  p->lam_hist[k] = st->lam_cur;
-  bool stop = false;
-  int rule = 0;
-  const int64_t kmax = p->kmax;
-  switch (p->stoprule) {
-    case AIRT_STOP_DP:  // check_stoprules.m:56-72
-      if (nrk <= p->taudelta || k >= kmax) {
-        stop = true;
-        rule = (k != kmax) ? 2 : 0;
-      }
-      break;
-    case AIRT_STOP_ME: {  // check_stoprules.m:74-94
-      const double np = sqrt(st->acc[2]);
-      const double dme = st->acc[3] / 2.0;
-      if (k > 0 && dme / np <= p->taudelta) {
-        stop = true;
-        rule = 3;
-      } else if (k >= kmax) {
-        stop = true;
-        rule = 0;
-      }
-      break;
-    }
-    case AIRT_STOP_NCP: {  // check_stoprules.m:97-150
-      double sum = 0.0;
-      for (int j = 0; j < p->ncp_cols; ++j) sum += p->ncc_col[j];
-      const double ncc = sum / p->ncp_cols;
-      const int ns = p->ncp_smooth;
-      double mx = -INFINITY, mxn = ncc;  // max(dk), max([dk(2:end); ncc]); NaN ignored
-      for (int i = 0; i < ns; ++i) mx = fmax(mx, p->dk[i]);
-      for (int i = 1; i < ns; ++i) mxn = fmax(mxn, p->dk[i]);
-      if (mx < mxn || k >= kmax) {
-        stop = true;
-        rule = (k != kmax) ? 1 : 0;
-      } else {
-        for (int i = 0; i + 1 < ns; ++i) p->dk[i] = p->dk[i + 1];
-        p->dk[ns - 1] = ncc;
-      }
-      break;
-    }
-    default:  // NONE, check_stoprules.m:153-161
-      if (k >= kmax) stop = true;
-  }
-  st->rmr_prev = st->acc[1];
-  for (int q = 0; q < 6; ++q) st->acc[q] = 0.0;
-  if (stop) {
-    st->stop = 1;
-    st->stoprule = rule;
-    st->finaliter = k;
-    st->lam_last = st->lam_cur;
-  } else {
-    const int kn = k + 1;
-    if (p->relax_kind == AIRT_RELAX_CONST) st->lam_cur = p->relaxpar;
-    else if (p->relax_kind == AIRT_RELAX_TABLE) st->lam_cur = p->relax_table[kn - 1];
-    st->iter = kn;
-  }
+  sirt_control(st, p);
 }
 
 __global__ void k_to_f32(int64_t n, const double *__restrict__ a, float *__restrict__ b,
@@ -598,13 +721,10 @@ void launch_fwd_t(Problem &P, const FwdOut &o) {
       k_sirt_fwd_dda<ME, true><<<gd, td, 0, s>>>(P.geom(), (int)P.m, P.x32.p, P.x32t.p, P.slow_y.p, o);
     return;
   }
-  const int L = vec_lanes_for(P.nnz, P.m);
-  const unsigned g = grid_for(P.m * L, kThreads, 4);
-  switch (L) {
-    case 8: k_sirt_fwd<8, ME><<<g, kThreads, 0, s>>>(P.m, P.rp.p, P.ci.p, P.rv.p, P.x32.p, o); break;
-    case 4: k_sirt_fwd<4, ME><<<g, kThreads, 0, s>>>(P.m, P.rp.p, P.ci.p, P.rv.p, P.x32.p, o); break;
-    default: k_sirt_fwd<2, ME><<<g, kThreads, 0, s>>>(P.m, P.rp.p, P.ci.p, P.rv.p, P.x32.p, o); break;
-  }
+  with_lanes(vec_lanes_for(P.nnz, P.m), [&](auto lanes) {
+    constexpr int L = decltype(lanes)::value;
+    k_sirt_fwd<L, ME><<<grid_for(P.m * L, kThreads, 4), kThreads, 0, s>>>(P.m, P.rp.p, P.ci.p, P.rv.p, P.x32.p, o);
+  });
 }
 
 void launch_fwd(Problem &P, const FwdOut &o, bool me) {
@@ -624,13 +744,10 @@ void launch_bwd_t(Problem &P, const UpdArgs &u) {
     AIRT_STREAM_LAUNCH((k_sirt_bwd_stream<MODE>), sa.ntiles, sa, u);
     return;
   }
-  const int L = vec_lanes_for(P.nnz, P.n);
-  const unsigned g = grid_for(P.n * L, kThreads, 4);
-  switch (L) {
-    case 8: k_sirt_bwd<8, MODE><<<g, kThreads, 0, s>>>(P.n, P.cp.p, P.ri.p, P.cv.p, P.mr32.p, u); break;
-    case 4: k_sirt_bwd<4, MODE><<<g, kThreads, 0, s>>>(P.n, P.cp.p, P.ri.p, P.cv.p, P.mr32.p, u); break;
-    default: k_sirt_bwd<2, MODE><<<g, kThreads, 0, s>>>(P.n, P.cp.p, P.ri.p, P.cv.p, P.mr32.p, u); break;
-  }
+  with_lanes(vec_lanes_for(P.nnz, P.n), [&](auto lanes) {
+    constexpr int L = decltype(lanes)::value;
+    k_sirt_bwd<L, MODE><<<grid_for(P.n * L, kThreads, 4), kThreads, 0, s>>>(P.n, P.cp.p, P.ri.p, P.cv.p, P.mr32.p, u);
+  });
 }
 
 void launch_bwd(Problem &P, const UpdArgs &u, int relax_kind, const double *Dfull) {
@@ -670,6 +787,68 @@ void launch_bwd(Problem &P, const UpdArgs &u, int relax_kind, const double *Dful
   }
   AIRT_LAUNCH_CHECK();
   prof_end(P, 1, e0);
+}
+
+// Matrices whose iterations run in one launch, and those that are small
+// enough for the variant with part of the matrix in registers.  Per iteration
+// (one launch with registers / without / launched kernels in a graph): 0.16 M
+// nonzeros 6.2 / 9.0 / 12.6 us, 0.94 M 9.2 / 10.8 / 17.4, 1.9 M 15.0 / 14.7 /
+// 20.8, 3.7 M 28 / 21 / 27, 6.3 M 58 / 38.5 / 38.8, 21 M - / 97 / 92.
+constexpr int64_t kPersistNnz = 6 << 20, kResidentNnz = 7 << 18;
+constexpr int64_t kPersistIters = 2048;  // iterations per launch
+constexpr int kPersistGrid = 160;        // CTAs at most (the kernel adds that many sums)
+
+template <int THREADS, int R>
+void run_persist(Problem &P, const FwdOut &fo, const UpdArgs &ua, int64_t kmax) {
+  cudaStream_t s = P.stream;
+  auto kernel = k_sirt_persist<THREADS, R>;
+  const unsigned grid = (unsigned)std::min(num_sms(), kPersistGrid);
+  // lanes per segment: the fewest vector loads in a row per lane, where a
+  // segment's fixed part (bounds, reduction, epilogue) counts as three
+  auto lanes = [&](int64_t nseg) {
+    const double avg = (double)P.nnz / (double)nseg;
+    int best = 2;
+    double cost = INFINITY;
+    for (int L = 2; L <= 32; L *= 2) {
+      const double c = std::ceil((double)nseg * L / ((double)grid * THREADS)) * (avg / (4.0 * L) + 3.0);
+      if (c < cost) {
+        cost = c;
+        best = L;
+      }
+    }
+    return best;
+  };
+  int occ = 0;
+  AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, 0));
+  AIRT_REQUIRE(occ >= 1, "the one-launch SIRT kernel cannot be resident");
+  P.pst_part.ensure(2 * grid);
+  P.pst_count.ensure(1);
+  PersistArgs a{};
+  a.rows = PersistDir{(int)P.m, P.rp.p, P.ci.p, P.rv.p, lanes(P.m)};
+  a.cols = PersistDir{(int)P.n, P.cp.p, P.ri.p, P.cv.p, lanes(P.n)};
+  a.b = fo.b;
+  a.M = fo.M;
+  a.mr32 = fo.mr32;
+  a.u = ua;
+  a.p = P.params.p;
+  a.part = P.pst_part.p;
+  a.count = P.pst_count.p;
+  a.err = P.err.p;
+  a.budget = g_persist_wait_budget;
+  if (!P.h_state) AIRT_CHECK_CUDA(cudaMallocHost(&P.h_state, 3 * sizeof(SirtState)));
+  for (int64_t it = 0; it < kmax; it = a.it1) {
+    a.it0 = (int)it;
+    a.it1 = (int)std::min(kmax, it + kPersistIters);
+    AIRT_CHECK_CUDA(cudaMemsetAsync(P.pst_count.p, 0, sizeof(unsigned), s));
+    void *args[] = {&a};
+    AIRT_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(THREADS), args, 0, s));
+    if (a.it1 == kmax) break;
+    int herr = 0;
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(P.h_state, P.state.p, sizeof(SirtState), cudaMemcpyDeviceToHost, s));
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(&herr, P.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+    if (herr || P.h_state->stop) break;
+  }
 }
 
 }  // namespace
@@ -716,6 +895,7 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
   const bool mfull = o.method == AIRT_CUSTOM && o.M && o.M_full;
   const bool dfull = o.method == AIRT_CUSTOM && o.D && o.D_full;
   if (o.method == AIRT_CUSTOM) {
+    P.wt_method = -1;
     AIRT_REQUIRE(!mfull || (double)m * (double)m <= 4e9,
                  "a full custom M of %lld x %lld does not fit the device", (long long)m,
                  (long long)m);
@@ -750,7 +930,7 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
     }
     AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
   } else {
-    compute_weights(P, o.method, P.M.p, P.D.p);
+    use_weights(P, o.method);
   }
 
   // vectors
@@ -817,7 +997,10 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
   P.params.upload(&prm, 1, s);
 
 
-  FwdOut fo{d_b, P.M.p, P.mr32.p, me ? P.rprev.p : nullptr, P.state.p};
+  // the control step runs in the forward pass unless NCP or a full M needs
+  // kernels between the two
+  const bool own_ctrl = ncp || mfull || m == 0;
+  FwdOut fo{d_b, P.M.p, P.mr32.p, me ? P.rprev.p : nullptr, P.state.p, own_ctrl ? nullptr : P.params.p};
   UpdArgs ua{};
   ua.D = P.D.p;
   ua.x64 = P.x64.p;
@@ -836,6 +1019,10 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
   ua.x32t = walks ? P.x32t.p : nullptr;
   ua.N = P.N;
 
+  // a small stored problem runs in one launch (persist.cuh)
+  const bool persist = !P.matrix_free && P.spmv_kind == 0 && !me && !dfull && !P.profiling &&
+                       o.relax_kind != AIRT_RELAX_LINE && o.kmax < INT32_MAX - 2 && m > 0 && n > 0 && kmax > 0 && P.nnz > 0 &&
+                       P.nnz <= kPersistNnz;
   // forward pass, and with NCP the periodogram of the new residual
   const double *Dfull = dfull ? P.Dfull.p : nullptr;
   auto fwd = [&]() {
@@ -850,37 +1037,44 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
       k_ncp_col<<<o.ncp_cols, 256, 0, s>>>(ncp_q, P.ncp_pk.p, P.ncp_col.p, &P.state.p->stop);
       AIRT_LAUNCH_CHECK();
     }
+    if (own_ctrl) {
+      k_sirt_ctrl<<<1, 32, 0, s>>>(P.state.p, P.params.p);
+      AIRT_LAUNCH_CHECK();
+    }
   };
   // initial residual and stop check (sirt.m:153-162)
-  fwd();
-  k_sirt_ctrl<<<1, 32, 0, s>>>(P.state.p, P.params.p);
-  AIRT_LAUNCH_CHECK();
+  if (persist && P.nnz <= kResidentNnz) run_persist<512, 3>(P, fo, ua, kmax);
+  else if (persist) run_persist<1024, 0>(P, fo, ua, kmax);
+  else fwd();
 
-  // main loop, enqueued in chunks; the flag of chunk c is read after chunk
-  // c+1 has been queued so the device never idles on the poll
+  // main loop, enqueued in chunks.  Without a data-dependent stopping rule
+  // every iteration runs: enqueue them all.  Otherwise the flag of a chunk is
+  // read once a later one is queued, so that the device never idles on the
+  // poll: the next one while chunks are short (a solve that stops early then
+  // has few iterations queued behind it), the one after it later, so that
+  // host-side stalls do not drain the queue.
   if (!P.h_state) AIRT_CHECK_CUDA(cudaMallocHost(&P.h_state, 3 * sizeof(SirtState)));
   cudaEvent_t ev[3];
   for (int q = 0; q < 3; ++q)
     AIRT_CHECK_CUDA(cudaEventCreateWithFlags(&ev[q], cudaEventDisableTiming));
-  // Without a data-dependent stopping rule every iteration runs: enqueue
-  // them all.  Otherwise poll the flag of chunk c once chunk c+2 is queued,
-  // so host-side stalls never drain the device queue.
   const bool poll = o.stoprule != AIRT_STOP_NONE;
   const int64_t chunk = 16;
-  const int lag = 2;
-  int64_t c = 0;
   // A full chunk is captured once as a CUDA graph and replayed: the kernel
   // arguments never change between iterations (all loop state lives in
   // device memory), so one graph serves the whole solve.  With per-launch
   // profiling on, kernels are launched one by one so each gets its events.
+  // It saves 2-3 us per iteration and costs about 0.25 ms, so it waits for a
+  // solve with graph_left iterations ahead and, where a rule may stop it,
+  // graph_after behind.
+  const int64_t graph_left = 128, graph_after = poll ? 48 : 0;
   cudaGraphExec_t chunk_graph = nullptr;
-  if (!P.profiling && kmax >= chunk) {
+  bool captured = P.profiling;
+  auto capture = [&]() {
     cudaGraph_t g = nullptr;
     AIRT_CHECK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int64_t j = 0; j < chunk; ++j) {
       launch_bwd(P, ua, o.relax_kind, Dfull);
       fwd();
-      k_sirt_ctrl<<<1, 32, 0, s>>>(P.state.p, P.params.p);
     }
     const cudaError_t ec = cudaStreamEndCapture(s, &g);
     if (ec == cudaSuccess && g) {
@@ -888,16 +1082,20 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
       cudaGraphDestroy(g);
     }
     cudaGetLastError();
-  }
-  for (int64_t it = 1; it <= kmax; ++c) {
-    const int64_t cnt = (kmax - it + 1 < chunk) ? (kmax - it + 1) : chunk;
+    captured = true;
+  };
+  int64_t c = 0;
+  for (int64_t it = 1; !persist && it <= kmax; ++c) {
+    const bool early = poll && c < 8;
+    const int64_t want = early ? (c < 4 ? 4 : 8) : chunk, left = kmax - it + 1;
+    const int64_t cnt = left < want ? left : want;
+    if (!captured && !early && it > graph_after && left >= graph_left) capture();
     if (cnt == chunk && chunk_graph) {
       AIRT_CHECK_CUDA(cudaGraphLaunch(chunk_graph, s));
     } else {
       for (int64_t j = 0; j < cnt; ++j) {
         launch_bwd(P, ua, o.relax_kind, Dfull);
         fwd();
-        k_sirt_ctrl<<<1, 32, 0, s>>>(P.state.p, P.params.p);
       }
     }
     AIRT_LAUNCH_CHECK();
@@ -906,20 +1104,21 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
     AIRT_CHECK_CUDA(cudaMemcpyAsync(P.h_state + (c % 3), P.state.p, sizeof(SirtState),
                                     cudaMemcpyDeviceToHost, s));
     AIRT_CHECK_CUDA(cudaEventRecord(ev[c % 3], s));
+    const int lag = early ? 1 : 2;
     if (c >= lag) {
       AIRT_CHECK_CUDA(cudaEventSynchronize(ev[(c - lag) % 3]));
       if (P.h_state[(c - lag) % 3].stop) break;
     }
   }
+  int herr = 0;
   AIRT_CHECK_CUDA(cudaMemcpyAsync(P.h_state, P.state.p, sizeof(SirtState), cudaMemcpyDeviceToHost, s));
+  AIRT_CHECK_CUDA(cudaMemcpyAsync(&herr, P.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
   if (chunk_graph) cudaGraphExecDestroy(chunk_graph);
   for (int q = 0; q < 3; ++q) cudaEventDestroy(ev[q]);
   const SirtState st = P.h_state[0];
-  int herr = 0;
-  AIRT_CHECK_CUDA(cudaMemcpy(&herr, P.err.p, sizeof(int), cudaMemcpyDeviceToHost));
   if (herr) {
-    set_error("a bounded device wait gave up (bulk copy did not complete)");
+    set_error("a bounded device wait gave up");
     throw Status{AIRT_ERR_TIMEOUT};
   }
   AIRT_REQUIRE(st.stop, "internal: SIRT loop ended without a stop");
@@ -986,17 +1185,54 @@ __global__ void k_dot2(int64_t n, const double *__restrict__ u, const double *__
     atomicAdd(out + 1, b);
   }
 }
-// w -= a * x
-__global__ void k_axmy(int64_t n, double a, const double *__restrict__ x, double *__restrict__ w) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    w[i] -= a * x[i];
-}
 __global__ void k_scale_by(int64_t n, double c, const double *__restrict__ w,
                            double *__restrict__ u) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     u[i] = w[i] * c;
+}
+
+// Lanczos vectors.  red holds the sums of a step, zeroed by the host:
+// red[0] = a_j, red[1] = b_(j+1)^2; prev the previous step's.
+// v = w / b (b > 0 by the caller; first step: v is given) and t = sd .* v.
+__global__ void k_lanczos_next(int64_t n, double inv_b, const double *__restrict__ sd,
+                               const double *__restrict__ w, double *__restrict__ v, double *__restrict__ t) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    double x = v[i];
+    if (w) v[i] = x = w[i] * inv_b;
+    t[i] = sd[i] * x;
+  }
+}
+// w = sd .* t - b * vprev (vprev null: first step), red[0] += v'*w.
+__global__ void __launch_bounds__(kThreads)
+    k_lanczos_a(int64_t n, double b, const double *__restrict__ sd, const double *__restrict__ t,
+                const double *__restrict__ vprev, const double *__restrict__ v, double *__restrict__ w,
+                double *__restrict__ red) {
+  double a = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    double x = sd[i] * t[i];
+    if (vprev) x -= b * vprev[i];
+    w[i] = x;
+    a += v[i] * x;
+  }
+  a = block_sum<kThreads>(a);
+  if (threadIdx.x == 0) atomicAdd(red, a);
+}
+// w -= red[0] * v, red[1] += w'*w.
+__global__ void __launch_bounds__(kThreads)
+    k_lanczos_b(int64_t n, const double *__restrict__ v, double *__restrict__ w, double *__restrict__ red) {
+  const double a = red[0];
+  double s = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const double x = w[i] - a * v[i];
+    w[i] = x;
+    s += x * x;
+  }
+  s = block_sum<kThreads>(s);
+  if (threadIdx.x == 0) atomicAdd(red + 1, s);
 }
 
 // Largest eigenvalue of the symmetric tridiagonal matrix with diagonal
@@ -1055,19 +1291,11 @@ double estimate_rho(Problem &P, const double *dM, const double *dD, double tol, 
   std::vector<double> h(n, 1.0 / std::sqrt((double)n));
   v.upload(h.data(), n, s);
   std::vector<double> alpha, beta{0.0};
-  double theta = 0.0, prev = 0.0;
-  auto dot = [&](const double *a, const double *b) {  // a.b
-    AIRT_CHECK_CUDA(cudaMemsetAsync(red.p, 0, 2 * sizeof(double), s));
-    k_dot2<<<gn, kThreads, 0, s>>>(n, a, b, red.p);
-    AIRT_LAUNCH_CHECK();
-    double hr[2];
-    AIRT_CHECK_CUDA(cudaMemcpyAsync(hr, red.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
-    return hr[0];
-  };
+  double theta = 0.0, prev = 0.0, inv_b = 0.0;
   for (int it = 0; it < std::max(maxit, 1); ++it) {
-    // w = S v - beta_j v_(j-1)
-    k_mul<<<gn, kThreads, 0, s>>>(n, sd.p, v.p, t.p);
+    // w = S v - beta_j v_(j-1), a_j = v'*w, w -= a_j v, b_(j+1) = ||w||; the
+    // host reads the two sums once per step
+    k_lanczos_next<<<gn, kThreads, 0, s>>>(n, inv_b, sd.p, it ? w.p : nullptr, v.p, t.p);
     if (m) {
       apply_operator(P, t.p, y.p, 0);
       k_mul<<<gm, kThreads, 0, s>>>(m, dM, y.p, y.p);
@@ -1075,23 +1303,23 @@ double estimate_rho(Problem &P, const double *dM, const double *dD, double tol, 
     } else {
       AIRT_CHECK_CUDA(cudaMemsetAsync(t.p, 0, n * sizeof(double), s));
     }
-    k_mul<<<gn, kThreads, 0, s>>>(n, sd.p, t.p, w.p);
-    if (it > 0) k_axmy<<<gn, kThreads, 0, s>>>(n, beta.back(), vprev.p, w.p);
+    AIRT_CHECK_CUDA(cudaMemsetAsync(red.p, 0, 2 * sizeof(double), s));
+    k_lanczos_a<<<gn, kThreads, 0, s>>>(n, beta.back(), sd.p, t.p, it ? vprev.p : nullptr, v.p, w.p, red.p);
+    k_lanczos_b<<<gn, kThreads, 0, s>>>(n, v.p, w.p, red.p);
     AIRT_LAUNCH_CHECK();
-    const double a = dot(v.p, w.p);
-    alpha.push_back(a);
-    k_axmy<<<gn, kThreads, 0, s>>>(n, a, v.p, w.p);
-    AIRT_LAUNCH_CHECK();
-    const double b = std::sqrt(std::fmax(dot(w.p, w.p), 0.0));
+    double hr[2];
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(hr, red.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+    alpha.push_back(hr[0]);
+    const double b = std::sqrt(std::fmax(hr[1], 0.0));
     theta = tridiag_max_eig(alpha, beta);
     if (!(b > 1e-14 * std::fmax(std::fabs(theta), 1e-300))) break;  // invariant subspace
     if (it >= 4 && std::fabs(theta - prev) <= tol * std::fabs(theta)) break;
     prev = theta;
     beta.push_back(b);
+    inv_b = 1.0 / b;
     std::swap(vprev.p, v.p);
     std::swap(vprev.n, v.n);
-    k_scale_by<<<gn, kThreads, 0, s>>>(n, 1.0 / b, w.p, v.p);
-    AIRT_LAUNCH_CHECK();
   }
   return theta;
 }

@@ -340,7 +340,19 @@ void row_sums_sq(Problem &P, double *out) {
   AIRT_LAUNCH_CHECK();
 }
 
-// dM (m) and dD (n) receive the diagonals; landweber gives ones.
+// dM (m) and dD (n) receive the diagonals; landweber gives ones.  P.M and P.D
+// keep a method's weights (they depend on the operator alone) until another
+// method's or a caller's own weights are put there (P.wt_method = -1).
+void compute_weights(Problem &P, int method, double *dM, double *dD);
+void use_weights(Problem &P, int method) {
+  P.M.ensure(P.m);
+  P.D.ensure(P.n);
+  if (P.wt_method == method) return;
+  P.wt_method = -1;
+  compute_weights(P, method, P.M.p, P.D.p);
+  P.wt_method = method;
+}
+
 void compute_weights(Problem &P, int method, double *dM, double *dD) {
   cudaStream_t s = P.stream;
   const int64_t m = P.m, n = P.n;
@@ -405,9 +417,9 @@ void apply_operator(Problem &P, const double *d_in, double *d_out, int transp) {
     return;
   }
   if (!transp)
-    spmv_plain(P.m, P.rp.p, P.ci.p, P.rv.p, d_in, d_out, s);
+    spmv_plain(P.m, P.nnz, P.rp.p, P.ci.p, P.rv.p, d_in, d_out, s);
   else
-    spmv_plain(P.n, P.cp.p, P.ri.p, P.cv.p, d_in, d_out, s);
+    spmv_plain(P.n, P.nnz, P.cp.p, P.ri.p, P.cv.p, d_in, d_out, s);
 }
 
 }  // namespace airt

@@ -6,6 +6,8 @@
 // with warp shuffles.  The group width is chosen from the mean segment length.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace airt {
@@ -344,6 +346,16 @@ inline int vec_lanes_for(int64_t nnz, int64_t nseg) {
   return 2;
 }
 
+// Calls f(std::integral_constant<int, lanes>) for lanes = 2, 4 or 8.
+template <class F>
+inline void with_lanes(int lanes, F &&f) {
+  switch (lanes) {
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    default: f(std::integral_constant<int, 2>{}); break;
+  }
+}
+
 template <int LANES>
 __global__ void __launch_bounds__(256, 4) k_spmv_plain(int64_t nseg, const int64_t *__restrict__ ptr,
                                                        const int *__restrict__ idx,
@@ -363,19 +375,13 @@ inline int lanes_for(int64_t nnz, int64_t nseg) {
   return 4;
 }
 
-inline void spmv_plain(int64_t nseg, const int64_t *ptr, const int *idx, const float *val,
+inline void spmv_plain(int64_t nseg, int64_t nnz, const int64_t *ptr, const int *idx, const float *val,
                        const double *x, double *y, cudaStream_t s) {
   if (nseg == 0) return;
-  int64_t nnz = 0;
-  AIRT_CHECK_CUDA(cudaMemcpyAsync(&nnz, ptr + nseg, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
-  const int L = vec_lanes_for(nnz, nseg);
-  const unsigned g = grid_for(nseg * L, 256, 4);
-  switch (L) {
-    case 8: k_spmv_plain<8><<<g, 256, 0, s>>>(nseg, ptr, idx, val, x, y); break;
-    case 4: k_spmv_plain<4><<<g, 256, 0, s>>>(nseg, ptr, idx, val, x, y); break;
-    default: k_spmv_plain<2><<<g, 256, 0, s>>>(nseg, ptr, idx, val, x, y); break;
-  }
+  with_lanes(vec_lanes_for(nnz, nseg), [&](auto lanes) {
+    constexpr int L = decltype(lanes)::value;
+    k_spmv_plain<L><<<grid_for(nseg * L, 256, 4), 256, 0, s>>>(nseg, ptr, idx, val, x, y);
+  });
   AIRT_LAUNCH_CHECK();
 }
 
