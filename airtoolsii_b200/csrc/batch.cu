@@ -837,7 +837,7 @@ void batch_destroy(Batch *B) {
   if (!B) return;
   cudaStream_t s = B->P.stream;
   if (s) cudaStreamSynchronize(s);
-  if (B->P.h_state) cudaFreeHost(B->P.h_state);
+  pinned_free(B->P.h_state);
   B->P.h_state = nullptr;
   delete B;
   if (s) cudaStreamDestroy(s);
@@ -1148,7 +1148,7 @@ void batch_sirt(Batch &B, int method, const double *lam_host, const double *d_b,
     }
     cudaGetLastError();
   }
-  if (!P.h_state) AIRT_CHECK_CUDA(cudaMallocHost(&P.h_state, 3 * sizeof(SirtState)));
+  ensure_h_state(P);
   int *hact = reinterpret_cast<int *>(P.h_state);  // 3 poll slots in the pinned mirror
   cudaEvent_t ev[3];
   for (int q = 0; q < 3; ++q) AIRT_CHECK_CUDA(cudaEventCreateWithFlags(&ev[q], cudaEventDisableTiming));

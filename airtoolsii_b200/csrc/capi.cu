@@ -86,7 +86,7 @@ static void free_problem(Problem *P) {
     cudaEventDestroy(it.second.second);
   }
   for (auto e : P->ev_pool) cudaEventDestroy(e);
-  if (P->h_state) cudaFreeHost(P->h_state);
+  pinned_free(P->h_state);
   cudaStream_t s = P->stream;
   delete P;
   if (s) cudaStreamDestroy(s);

@@ -48,6 +48,17 @@ void set_error(const char *fmt, ...);
 // device were out of memory.
 extern int g_alloc_fail_countdown;
 
+// Device memory for DevBuf (pool.cu): blocks that are given up are kept for
+// the next allocation of about their size.  device_alloc returns null when
+// the device is out of memory (*err then holds CUDA's error).  device_free
+// waits for the device, as cudaFree does, so a kept block is idle.
+void *device_alloc(size_t bytes, cudaError_t *err);
+void device_free(void *p);
+// One page-locked buffer of kPinnedBytes, kept likewise.
+constexpr size_t kPinnedBytes = 1024;
+void *pinned_alloc(cudaError_t *err);
+void pinned_free(void *p);
+
 template <typename T>
 struct DevBuf {
   T *p = nullptr;
@@ -71,7 +82,7 @@ struct DevBuf {
   }
   ~DevBuf() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p) device_free(p);
     p = nullptr;
     n = 0;
   }
@@ -84,9 +95,9 @@ struct DevBuf {
       set_error("cudaMalloc of %zu bytes failed: injected allocation failure (test hook)", bytes);
       throw Status{AIRT_ERR_OOM};
     }
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-      p = nullptr;
+    cudaError_t e = cudaSuccess;
+    p = static_cast<T *>(device_alloc(bytes, &e));
+    if (!p) {
       set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
       throw Status{AIRT_ERR_OOM};
     }
@@ -260,7 +271,7 @@ struct Problem {
   DevBuf<double> pst_part;     // one-launch SIRT (persist.cuh): partial sums, barrier counter
   DevBuf<unsigned> pst_count;
   DevBuf<int> save_slot;
-  SirtState *h_state = nullptr;  // pinned mirror
+  SirtState *h_state = nullptr;  // pinned mirror (3 entries)
 
   // instrumentation
   bool profiling = false;
@@ -297,6 +308,14 @@ struct Problem {
 };
 
 // ---------------------------------------------------------------- helpers
+inline void ensure_h_state(Problem &P) {
+  static_assert(3 * sizeof(SirtState) <= kPinnedBytes, "pinned mirror");
+  if (P.h_state) return;
+  cudaError_t e = cudaSuccess;
+  P.h_state = static_cast<SirtState *>(pinned_alloc(&e));
+  AIRT_CHECK_CUDA(e);
+}
+
 inline int num_sms() {
   static int sms = 0;
   if (!sms) {

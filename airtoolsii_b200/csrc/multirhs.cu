@@ -438,7 +438,7 @@ void multi_pass(Problem &P, const airt_sirt_opts &o, int K0, const double *d_B, 
     cudaGetLastError();
   };
   capture();
-  if (!P.h_state) AIRT_CHECK_CUDA(cudaMallocHost(&P.h_state, 3 * sizeof(SirtState)));
+  ensure_h_state(P);
   static_assert(sizeof(MultiState) <= sizeof(SirtState), "poll slots");
   MultiState *hs = reinterpret_cast<MultiState *>(P.h_state);  // 3 slots in the pinned mirror
   cudaEvent_t ev[3];

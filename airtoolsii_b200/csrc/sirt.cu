@@ -835,7 +835,7 @@ void run_persist(Problem &P, const FwdOut &fo, const UpdArgs &ua, int64_t kmax) 
   a.count = P.pst_count.p;
   a.err = P.err.p;
   a.budget = g_persist_wait_budget;
-  if (!P.h_state) AIRT_CHECK_CUDA(cudaMallocHost(&P.h_state, 3 * sizeof(SirtState)));
+  ensure_h_state(P);
   for (int64_t it = 0; it < kmax; it = a.it1) {
     a.it0 = (int)it;
     a.it1 = (int)std::min(kmax, it + kPersistIters);
@@ -1053,7 +1053,7 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
   // poll: the next one while chunks are short (a solve that stops early then
   // has few iterations queued behind it), the one after it later, so that
   // host-side stalls do not drain the queue.
-  if (!P.h_state) AIRT_CHECK_CUDA(cudaMallocHost(&P.h_state, 3 * sizeof(SirtState)));
+  ensure_h_state(P);
   cudaEvent_t ev[3];
   for (int q = 0; q < 3; ++q)
     AIRT_CHECK_CUDA(cudaEventCreateWithFlags(&ev[q], cudaEventDisableTiming));

@@ -171,8 +171,9 @@ bool build_tiles(Problem &P, const int64_t *d_ptr, int64_t nseg, DevBuf<int> &ti
   return true;
 }
 
+// Tile tables of the streamed kernels, where those were asked for.
 void finalize_matrix(Problem &P) {
-  P.stream_ok = build_tiles(P, P.rp.p, P.m, P.rtiles, P.nrtiles) &&
+  P.stream_ok = P.spmv_kind == 1 && build_tiles(P, P.rp.p, P.m, P.rtiles, P.nrtiles) &&
                 build_tiles(P, P.cp.p, P.n, P.ctiles, P.nctiles);
 }
 
