@@ -10,20 +10,30 @@
 // separates levels.  Each pixel therefore sees the same update sequence, and
 // each dot product reads the same values, as in the sequential sweep.
 //
-// The sweep runs as one cooperative launch over all SMs with one warp per
-// step: the steps, sorted by level, are dealt round-robin to every warp of
-// the grid, and a step waits only for its predecessors -- the last earlier
-// step that touched each of its pixels -- through per-step completion
-// stamps in global memory (release store after the step's x writes, acquire
-// loads before its gathers).  The chain of levels is the critical path; no
-// grid-wide barrier separates levels.  Each wait is bounded: on expiry the
-// kernel raises an error flag, every warp leaves, and the host reports
-// AIRT_ERR_TIMEOUT.
+// The sweep runs as one launch over all SMs with one warp per step: the steps,
+// sorted by level, are dealt round-robin to every warp of the grid, and a step
+// waits only until each of its pixels has been written by the earlier steps
+// that touch it.  A pixel is a 16-byte word {x, writes so far}, read and
+// written by 128-bit accesses, and the schedule holds for every entry how
+// many writes must precede it: the poll that finds a pixel ready has its value
+// already, and a step publishes its pixels with the stores that write them --
+// no completion flags, no fences, no gather after the wait.  The chain of
+// levels is the critical path; no grid-wide barrier separates levels.  Each
+// wait is bounded: on expiry the kernel raises an error flag, every warp
+// leaves, and the host reports AIRT_ERR_TIMEOUT.
+//
+// Bound: the latency of a level (scattered 128-bit stores, poll, sum), 1.6 us
+// with 256 entries per row.  Per sweep, against completion flags per step with
+// fences and a gather after the wait: N = 64, 30 angles 0.71 -> 0.30 ms;
+// N = 128, 90 angles 1.80 -> 0.74 ms; N = 256, 180 angles 4.58 -> 1.81 ms;
+// N = 400, 90 angles (rows past the 512 entries kept in registers) 10.1 -> 7.5.
 //
 // The whole-vector box projection after every row (art.m:279-284) is
 // equivalent to clamping x0 once right after the first row step and the
 // row's support after every later step: once x is feasible only the updated
 // entries can leave the box.  The first step reads x0 unclamped.
+#include <cub/device/device_radix_sort.cuh>
+
 #include <algorithm>
 #include <cmath>
 #include <numeric>
@@ -45,6 +55,7 @@ struct KaczArgs {
   double lam;
   const double *lam_tab;  // per step of this sweep, or null
   double *x;
+  ulonglong2 *xv;         // {x bits, writes in this sweep} of every pixel
   int lbk, ubk;
   double lb, ub;
   const double *lbv, *ubv;
@@ -58,113 +69,252 @@ __device__ __forceinline__ double clampv(double v, int64_t j, const KaczArgs &a)
   return v;
 }
 
+// 0: no bounds, 1: scalar bounds only, 2: a vector among them.
+__device__ __forceinline__ int clamp_mode(const KaczArgs &a) {
+  if (a.lbk == AIRT_BOUND_VECTOR || a.ubk == AIRT_BOUND_VECTOR) return 2;
+  return a.lbk != AIRT_BOUND_NONE || a.ubk != AIRT_BOUND_NONE;
+}
+
+// Scalar bounds without a branch (a NaN takes the bound, as fmax and fmin do).
+__device__ __forceinline__ double clamp_scalar(double v, const KaczArgs &a) {
+  v = a.lbk != AIRT_BOUND_NONE && !(v >= a.lb) ? a.lb : v;
+  return a.ubk != AIRT_BOUND_NONE && !(v <= a.ub) ? a.ub : v;
+}
+
 // Test hook: a cycle budget for the bounded waits of the sweep kernel and
 // an injected stall (the first step waits for a stamp that no step writes),
 // so that a test can make a wait run out.  Defaults: ~2 s, no stall.
 long long g_kacz_wait_budget = 4000000000ll;
 int g_kacz_inject_stall = 0;
 
-constexpr int kDagCache = 16;  // entries per lane kept in registers (rows <= 512)
-// Warps per CTA of the sweep kernel (one CTA per SM) and the pause between
-// two polls of an unfinished predecessor (0: none).
-#ifndef AIRT_KACZ_WARPS
-#define AIRT_KACZ_WARPS 8
-#endif
-#ifndef AIRT_KACZ_BACKOFF_NS
-#define AIRT_KACZ_BACKOFF_NS 0
-#endif
-constexpr int kDagThreads = 32 * AIRT_KACZ_WARPS;
+constexpr int kDagThreads = 256;  // eight warps per CTA
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+// 128-bit relaxed accesses: one pixel's value and write count together.
+struct Pixels {
+  ulonglong2 *xv;
+  __device__ __forceinline__ ulonglong2 load(int j) const {
+    ulonglong2 v;
+    asm volatile(
+        "{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+        : "=l"(v.x), "=l"(v.y)
+        : "l"(xv + j)
+        : "memory");
+    return v;
+  }
+  // load_if leaves v alone and store_if does nothing unless `on`; predicated,
+  // so that a sequence of them is not cut by branches
+  __device__ __forceinline__ void load_if(bool on, int j, ulonglong2 &v) const {
+    asm volatile(
+        "{ .reg .b128 t; .reg .pred p; setp.ne.s32 p, %3, 0; mov.b128 t, {%0, %1};"
+        "  @p ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+        : "+l"(v.x), "+l"(v.y)
+        : "l"(xv + j), "r"((int)on)
+        : "memory");
+  }
+  __device__ __forceinline__ void store_if(bool on, int j, double x, unsigned long long writes) const {
+    asm volatile(
+        "{ .reg .b128 t; .reg .pred p; setp.ne.s32 p, %3, 0; mov.b128 t, {%1, %2};"
+        "  @p st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(xv + j),
+        "l"(__double_as_longlong(x)), "l"(writes), "r"((int)on)
+        : "memory");
+  }
+};
+// Bounded wait of one thread: true while it may go on polling.
+struct KaczWait {
+  int *err;
+  long long budget, t0;
+  unsigned n = 0;
+  __device__ __forceinline__ bool more() {
+    if (++n % 32) return true;
+    if (*(volatile int *)err) return false;
+    if (clock64() - t0 > budget) {
+      atomicExch(err, 1);
+      return false;
+    }
+    return true;
+  }
+};
+
+struct SweepArgs {
+  int nsteps;
+  const ArtStep *steps;
+  const uint2 *ent;
+  int *err;
+  long long budget;
+  int stall;
+};
+
+// One step's operands: the entries of its row (E per lane; longer rows are
+// read past them one by one), b, and lambda over the squared norm.
+template <int E>
+struct KaczRow {
+  ArtStep st;
+  int cj[E];
+  float cv[E];
+  unsigned cn[E];
+  double bi, lam;
+};
+
+__device__ __forceinline__ ArtStep load_step(const SweepArgs &w, int q) {
+  ArtStep s{0, 0, 0, 0, 0, -1};
+  if (q < w.nsteps) {
+    const longlong2 a = __ldg(reinterpret_cast<const longlong2 *>(w.steps + q));
+    const int4 b = __ldg(reinterpret_cast<const int4 *>(w.steps + q) + 1);
+    s = ArtStep{a.x, a.y, b.x, b.y, b.z, b.w};
+  }
+  return s;
 }
 
-// One Kaczmarz sweep in the level-sorted step order: warp w of the grid
-// (consecutive warps on different SMs) runs steps w, w+W, w+2W, ... ; step q
-// waits until done[pred] >= stamp for each of its predecessors
-// preds[pred_ptr[q] .. pred_ptr[q+1]) (indices into the same order), then
-// computes exactly what the sequential sweep computes for its row and
-// publishes done[q] = stamp.  The row's indices, values, b and the norm are
-// loaded before the wait; x is read through L2 (other SMs wrote it).
-__global__ void __launch_bounds__(kDagThreads, 1)
-    k_kacz_dag(int nsteps, const int *__restrict__ steps, const int *__restrict__ step_pos,
-               const int *__restrict__ pred_ptr, const int *__restrict__ preds, unsigned stamp,
-               unsigned *__restrict__ done, int *__restrict__ err, long long budget, int stall,
-               KaczArgs a) {
+template <int E>
+__device__ __forceinline__ void load_row(const SweepArgs &w, const KaczArgs &a, const ArtStep &st, int lane,
+                                         KaczRow<E> &r) {
+  r.st = st;
+#pragma unroll
+  for (int u = 0; u < E; ++u) {
+    const int e = lane + 32 * u;
+    r.cj[u] = 0;
+    r.cv[u] = 0.f;
+    r.cn[u] = 0;
+    if (e < st.len) {
+      const uint2 p = __ldg(w.ent + st.off + e);
+      r.cj[u] = (int)p.x;
+      r.cn[u] = p.y;
+      r.cv[u] = __ldg(a.rv + st.s0 + e);
+    }
+  }
+  r.bi = r.lam = 0.0;
+  if (st.len) {
+    r.bi = __ldg(a.b + st.row);
+    // the division leaves the chain of the sweep
+    r.lam = (a.lam_tab ? __ldg(a.lam_tab + st.pos) : a.lam) / __ldg(a.nrm + st.row);
+  }
+}
+
+// Runs one step on the pixels px.  Its loads, sums and stores are free of
+// branches: with one per entry they ran one after the other (3.4 ms per sweep
+// at N = 256, 180 angles instead of 1.7).  The wait has two parts: a cheap one on the
+// entry whose previous writer comes last (rep), until that writer's own
+// predecessor is done, and then polls of all entries; with every waiting warp
+// polling all of its entries the polls would take bandwidth from the steps
+// that run.  Returns false when a wait ran out.
+template <int E>
+__device__ __forceinline__ bool kacz_step(const SweepArgs &w, const KaczArgs &a, const Pixels &px, KaczRow<E> &r,
+                                          int lane, bool stalled, int clamp) {
+  const ArtStep &st = r.st;
+  const int mine = min(E, (st.len - lane + 31) >> 5);  // entries of this lane
+  const unsigned all = mine > 0 ? (1u << mine) - 1u : 0u;
+  unsigned waiting = all;
+  // the test hook makes the first step wait for a write that never comes
+  if (stalled && lane == 0) r.cn[0] += 1;
+  KaczWait wait{w.err, w.budget, clock64()};
+  bool ok = true;
+  if (st.rep >= 0) {
+    const uint2 p = __ldg(w.ent + st.off + st.rep);
+    while ((unsigned)px.load((int)p.x).y + 1u < p.y && ok) ok = wait.more();
+  }
+  ulonglong2 v[E];
+#pragma unroll
+  for (int u = 0; u < E; ++u) v[u] = make_ulonglong2(0ull, 0ull);
+  while (ok && waiting) {
+#pragma unroll
+    for (int u = 0; u < E; ++u) px.load_if(waiting >> u & 1u, r.cj[u], v[u]);
+    unsigned ready = 0;
+#pragma unroll
+    for (int u = 0; u < E; ++u) ready |= ((unsigned)v[u].y == r.cn[u] ? 1u : 0u) << u;
+    waiting = all & ~ready;
+    if (waiting) ok = wait.more();
+  }
+  double acc = 0.0, acc1 = 0.0;
+#pragma unroll
+  for (int u = 0; u < E; u += 2) {  // entries the lane does not have are zero
+    acc = fma((double)r.cv[u], __longlong_as_double((long long)v[u].x), acc);
+    acc1 = fma((double)r.cv[u + 1], __longlong_as_double((long long)v[u + 1].x), acc1);
+  }
+  acc += acc1;
+  for (int e = lane + 32 * E; ok && e < st.len; e += 32) {
+    const uint2 p = __ldg(w.ent + st.off + e);
+    ulonglong2 o = px.load((int)p.x);
+    while ((unsigned)o.y != p.y && ok) {
+      ok = wait.more();
+      o = px.load((int)p.x);
+    }
+    acc = fma((double)__ldg(a.rv + st.s0 + e), __longlong_as_double((long long)o.x), acc);
+  }
+  if (!__all_sync(0xffffffffu, ok)) return false;
+  acc = warp_sum(acc);
+  const double c = r.lam * (r.bi - acc);
+  double xn[E];
+#pragma unroll
+  for (int u = 0; u < E; ++u) {
+    xn[u] = __dadd_rn(__longlong_as_double((long long)v[u].x), __dmul_rn(c, (double)r.cv[u]));
+    if (clamp == 1) xn[u] = clamp_scalar(xn[u], a);
+    if (clamp == 2) xn[u] = clampv(xn[u], r.cj[u], a);
+  }
+#pragma unroll
+  for (int u = 0; u < E; ++u) px.store_if(all >> u & 1u, r.cj[u], xn[u], r.cn[u] + 1ull);
+  for (int e = lane + 32 * E; e < st.len; e += 32) {
+    const int k = (int)__ldg(&w.ent[st.off + e].x);
+    const ulonglong2 o = px.load(k);
+    double x = __dadd_rn(__longlong_as_double((long long)o.x), __dmul_rn(c, (double)__ldg(a.rv + st.s0 + e)));
+    if (clamp) x = clampv(x, k, a);
+    px.store_if(true, k, x, o.y + 1ull);
+  }
+  return true;
+}
+
+// One Kaczmarz sweep in the level-sorted step order over all SMs: warp w of the grid (consecutive warps on different SMs)
+// runs steps w, w+W, w+2W, ... .
+__global__ void __launch_bounds__(kDagThreads, 1) k_kacz_sweep(SweepArgs w, KaczArgs a) {
   const int lane = threadIdx.x & 31;
   const int W = gridDim.x * (blockDim.x >> 5);
-  const int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const bool clamp = a.lbk != AIRT_BOUND_NONE || a.ubk != AIRT_BOUND_NONE;
-  for (int q = w; q < nsteps; q += W) {
-    const int row = __ldg(steps + q);
-    const int64_t s0 = __ldg(a.rp + row), s1 = __ldg(a.rp + row + 1);
-    const int64_t e0 = s0 + lane;
-    int cj[kDagCache];
-    float cv[kDagCache];
-#pragma unroll
-    for (int u = 0; u < kDagCache; ++u) {
-      const int64_t e = e0 + 32 * u;
-      cj[u] = e < s1 ? __ldg(a.ci + e) : -1;
-      cv[u] = e < s1 ? __ldg(a.rv + e) : 0.f;
-    }
-    const double bi = __ldg(a.b + row), ni = __ldg(a.nrm + row);
-    const double lam = a.lam_tab ? __ldg(a.lam_tab + __ldg(step_pos + q)) : a.lam;
-    // wait for the predecessors (each lane polls its share of them)
-    const int p0 = __ldg(pred_ptr + q), p1 = __ldg(pred_ptr + q + 1);
-    bool ok = true;
-    const long long t0 = clock64();
-    for (int pi = p0 + lane; ok && pi < p1 + (stall && q == 0 ? 1 : 0); pi += 32) {
-      const unsigned *f = pi < p1 ? done + __ldg(preds + pi) : done + q;  // stall: own stamp
-      const unsigned want = pi < p1 ? stamp : stamp + 1u;
-      while (ld_acquire_u32(f) < want) {
-        if (AIRT_KACZ_BACKOFF_NS > 0) __nanosleep(AIRT_KACZ_BACKOFF_NS);
-        if (*(volatile int *)err) {
-          ok = false;
-          break;
-        }
-        if (clock64() - t0 > budget) {
-          atomicExch(err, 1);
-          ok = false;
-          break;
-        }
-      }
-    }
-    if (!__all_sync(0xffffffffu, ok)) return;
-    // gathers (through L2) and the dot product in the order of the plain
-    // strided loop
-    double cx[kDagCache];
-#pragma unroll
-    for (int u = 0; u < kDagCache; ++u) cx[u] = cj[u] >= 0 ? __ldcg(a.x + cj[u]) : 0.0;
-    double acc = 0.0;
-#pragma unroll
-    for (int u = 0; u < kDagCache; ++u)
-      if (cj[u] >= 0) acc = fma((double)cv[u], cx[u], acc);
-    for (int64_t e = e0 + 32 * kDagCache; e < s1; e += 32)
-      acc = fma((double)__ldg(a.rv + e), __ldcg(a.x + __ldg(a.ci + e)), acc);
-    acc = warp_sum(acc);
-    const double c = __ddiv_rn(__dmul_rn(lam, __dsub_rn(bi, acc)), ni);
-#pragma unroll
-    for (int u = 0; u < kDagCache; ++u)
-      if (cj[u] >= 0) {
-        double v = __dadd_rn(cx[u], __dmul_rn(c, (double)cv[u]));
-        if (clamp) v = clampv(v, cj[u], a);
-        __stcg(a.x + cj[u], v);
-      }
-    for (int64_t e = e0 + 32 * kDagCache; e < s1; e += 32) {
-      const int j = __ldg(a.ci + e);
-      double v = __dadd_rn(__ldcg(a.x + j), __dmul_rn(c, (double)__ldg(a.rv + e)));
-      if (clamp) v = clampv(v, j, a);
-      __stcg(a.x + j, v);
-    }
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) st_release_u32(done + q, stamp);
+  const int clamp = clamp_mode(a);
+  for (int q = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; q < w.nsteps; q += W) {
+    KaczRow<16> r;
+    load_row(w, a, load_step(w, q), lane, r);
+    if (!kacz_step(w, a, Pixels{a.xv}, r, lane, w.stall && q == 0, clamp)) return;
   }
+}
+
+// xv = {x, 0}; and back: x from xv, the write counts zeroed for the next sweep.
+__global__ void k_pack_pixels(int n, const double *__restrict__ x, ulonglong2 *__restrict__ xv) {
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    xv[j] = make_ulonglong2((unsigned long long)__double_as_longlong(x[j]), 0ull);
+}
+__global__ void k_unpack_pixels(int n, double *__restrict__ x, ulonglong2 *__restrict__ xv) {
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    ulonglong2 *p = xv + j;
+    x[j] = __longlong_as_double((long long)p->x);
+    p->y = 0ull;
+  }
+}
+
+// Ranks of an order's entries: the pixels in the order of the steps, the start
+// of every pixel's run after a stable sort by pixel, and the distance from it.
+__global__ void k_order_pixels(int64_t nsteps, const int *__restrict__ order, const int64_t *__restrict__ toff,
+                               const int64_t *__restrict__ rp, const int *__restrict__ ci,
+                               unsigned *__restrict__ key, unsigned *__restrict__ at) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t t = w; t < nsteps; t += nw) {
+    const int64_t s0 = rp[order[t]], len = rp[order[t] + 1] - s0;
+    for (int64_t e = lane; e < len; e += 32) {
+      key[toff[t] + e] = (unsigned)ci[s0 + e];
+      at[toff[t] + e] = (unsigned)(toff[t] + e);
+    }
+  }
+}
+__global__ void k_run_starts(int64_t cnt, const unsigned *__restrict__ key, unsigned *__restrict__ start) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < cnt;
+       q += (int64_t)gridDim.x * blockDim.x)
+    if (q == 0 || key[q] != key[q - 1]) start[key[q]] = (unsigned)q;
+}
+__global__ void k_ranks(int64_t cnt, const unsigned *__restrict__ key,
+                        const unsigned *__restrict__ at, const unsigned *__restrict__ start,
+                        uint2 *__restrict__ ent) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < cnt;
+       q += (int64_t)gridDim.x * blockDim.x)
+    ent[at[q]] = make_uint2(key[q], (unsigned)q - start[key[q]]);
 }
 
 // Clamp x0 everywhere except on the support of the first row, whose step
@@ -231,58 +381,72 @@ uint64_t order_key(const int64_t *order, int64_t nsteps) {
   return h ? h : 1;
 }
 
-// Level schedule of a row order (see the file comment): steps sorted by
-// level (stable), each with the distinct last earlier writers of its pixels
-// as predecessors, given as indices into the sorted order.
-void build_schedule(const std::vector<int64_t> &hrp, const std::vector<int> &hci,
-                    const int64_t *order, int64_t nsteps, int64_t n, Schedule &S,
-                    cudaStream_t s) {
-  std::vector<int> level(nsteps), last(n, -1), seen(nsteps, -1);
-  std::vector<int64_t> tptr(nsteps + 1, 0);
-  std::vector<int> tpred;
+// Level schedule of a row order (see the file comment): the levels on the
+// host, the entries' ranks on the device.
+void build_schedule(Problem &P, const std::vector<int64_t> &hrp, const std::vector<int> &hci,
+                    const int64_t *order, int64_t nsteps, int64_t n, Schedule &S, cudaStream_t s) {
+  std::vector<int> level(nsteps), last(n, -1), rept(nsteps), ord(nsteps);
+  std::vector<int64_t> toff(nsteps + 1, 0);
   int maxlev = -1;
   for (int64_t t = 0; t < nsteps; ++t) {
-    const int64_t row = order[t];
-    int L = 0;
-    for (int64_t e = hrp[row]; e < hrp[row + 1]; ++e) {
-      const int w = last[hci[e]];
-      if (w >= 0 && seen[w] != (int)t) {
-        seen[w] = (int)t;
-        tpred.push_back(w);
-        L = std::max(L, level[w] + 1);
+    const int64_t row = order[t], e0 = hrp[row], e1 = hrp[row + 1];
+    int L = -1, at = -1;  // highest level that wrote one of the row's pixels
+    for (int64_t e = e0; e < e1; ++e) {
+      const int v = last[hci[e]];
+      if (v > L) {
+        L = v;
+        at = (int)(e - e0);
       }
     }
-    tptr[t + 1] = (int64_t)tpred.size();
+    ++L;
+    for (int64_t e = e0; e < e1; ++e) last[hci[e]] = L;
     level[t] = L;
-    for (int64_t e = hrp[row]; e < hrp[row + 1]; ++e) last[hci[e]] = (int)t;
+    rept[t] = at;
+    ord[t] = (int)row;
+    toff[t + 1] = toff[t] + (e1 - e0);
     maxlev = std::max(maxlev, L);
   }
   S.nlev = maxlev + 1;
   S.nsteps = nsteps;
-  std::vector<int> ptr(S.nlev + 1, 0), steps(nsteps), pos(nsteps), qof(nsteps);
+  const int64_t cnt = toff[nsteps];
+  AIRT_REQUIRE(cnt < (int64_t)UINT32_MAX, "the row order visits too many entries");
+  std::vector<int> ptr(S.nlev + 1, 0);
+  std::vector<ArtStep> steps(nsteps);
   for (int64_t t = 0; t < nsteps; ++t) ++ptr[level[t] + 1];
   for (int L = 0; L < S.nlev; ++L) ptr[L + 1] += ptr[L];
   for (int64_t t = 0; t < nsteps; ++t) {
-    const int q = ptr[level[t]]++;
-    steps[q] = (int)order[t];
-    pos[q] = (int)t;
-    qof[t] = q;
-  }
-  std::vector<int> pptr(nsteps + 1, 0), preds(tpred.size());
-  for (int64_t q = 0; q < nsteps; ++q) {
-    const int t = pos[q];
-    pptr[q + 1] = pptr[q] + (int)(tptr[t + 1] - tptr[t]);
-  }
-  for (int64_t q = 0; q < nsteps; ++q) {
-    const int t = pos[q];
-    int o = pptr[q];
-    for (int64_t k = tptr[t]; k < tptr[t + 1]; ++k) preds[o++] = qof[tpred[k]];
+    const int64_t row = order[t];
+    steps[ptr[level[t]]++] =
+        ArtStep{hrp[row], toff[t], (int)(hrp[row + 1] - hrp[row]), (int)row, (int)t, rept[t]};
   }
   S.steps.upload(steps.data(), nsteps, s);
-  S.pos.upload(pos.data(), nsteps, s);
-  S.pred_ptr.upload(pptr.data(), nsteps + 1, s);
-  if (preds.empty()) S.preds.ensure(1);
-  else S.preds.upload(preds.data(), preds.size(), s);
+  S.ent.ensure(cnt);
+  if (cnt) {
+    DevBuf<int> dord;
+    DevBuf<int64_t> dtoff;
+    DevBuf<unsigned> key, key2, at, at2, start;
+    DevBuf<unsigned char> tmp;
+    dord.upload(ord.data(), nsteps, s);
+    dtoff.upload(toff.data(), nsteps + 1, s);
+    key.ensure(cnt);
+    key2.ensure(cnt);
+    at.ensure(cnt);
+    at2.ensure(cnt);
+    start.ensure(n);
+    k_order_pixels<<<grid_for(nsteps * 32, 256), 256, 0, s>>>(nsteps, dord.p, dtoff.p, P.rp.p, P.ci.p, key.p, at.p);
+    AIRT_LAUNCH_CHECK();
+    int bits = 1;
+    while (bits < 31 && (1ll << bits) < n) ++bits;
+    size_t need = 0;
+    AIRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, need, key.p, key2.p, at.p, at2.p, cnt, 0, bits, s));
+    tmp.ensure(need);
+    AIRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, need, key.p, key2.p, at.p, at2.p, cnt, 0, bits, s));
+    const unsigned g = grid_for(cnt, 256);
+    k_run_starts<<<g, 256, 0, s>>>(cnt, key2.p, start.p);
+    k_ranks<<<g, 256, 0, s>>>(cnt, key2.p, at2.p, start.p, S.ent.p);
+    AIRT_LAUNCH_CHECK();
+  }
+  AIRT_CHECK_CUDA(cudaStreamSynchronize(s));  // the host vectors and work space end here
 }
 
 }  // namespace
@@ -378,7 +542,7 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
   }
   if (!per_sweep_sched && need_pattern) {
     S.key = 0;
-    build_schedule(hrp, hci, order.data(), per_sweep, n, S, s);
+    build_schedule(P, hrp, hci, order.data(), per_sweep, n, S, s);
     S.key = key;
   }
 
@@ -390,14 +554,13 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
     AIRT_CHECK_CUDA(cudaMemsetAsync(P.x64.p, 0, n * sizeof(double), s));
   if (o.lb_kind == AIRT_BOUND_VECTOR) P.lbv.upload(o.lbv, n, s);
   if (o.ub_kind == AIRT_BOUND_VECTOR) P.ubv.upload(o.ubv, n, s);
-  // sweep kernel: completion stamps of the steps, error flag, grid size
-  DevBuf<unsigned> done;
-  done.ensure(std::max<int64_t>(per_sweep, 1));
-  AIRT_CHECK_CUDA(cudaMemsetAsync(done.p, 0, std::max<int64_t>(per_sweep, 1) * sizeof(unsigned), s));
+  // sweep kernel: pixels with their write counts, error flag, grid size
+  DevBuf<ulonglong2> xv;
+  xv.ensure(std::max<int64_t>(n, 1));
   P.err.ensure(1);
   AIRT_CHECK_CUDA(cudaMemsetAsync(P.err.p, 0, sizeof(int), s));
   int occ = 0;
-  AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kacz_dag, kDagThreads, 0));
+  AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kacz_sweep, kDagThreads, 0));
   AIRT_REQUIRE(occ >= 1, "the Kaczmarz sweep kernel cannot be resident");
   const int dag_grid = num_sms();
   const long long budget = g_kacz_wait_budget;
@@ -416,6 +579,7 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
   a.nrm = nrm.p;
   a.lam = o.relaxpar;
   a.x = P.x64.p;
+  a.xv = xv.p;
   a.lbk = o.lb_kind;
   a.ubk = o.ub_kind;
   a.lb = o.lb;
@@ -473,7 +637,7 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
   double lam_last = o.relaxpar;
   for (int64_t k = 1; !st.stop; ++k) {
     const int64_t *ord = order.data() + (per_sweep_sched ? (k - 1) * per_sweep : 0);
-    if (per_sweep_sched) build_schedule(hrp, hci, ord, per_sweep, n, S, s);
+    if (per_sweep_sched) build_schedule(P, hrp, hci, ord, per_sweep, n, S, s);
     if (k == 1 && bounded && per_sweep > 0) {
       const int64_t r0 = ord[0];
       int64_t rr[2];
@@ -485,12 +649,12 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
     }
     a.lam_tab = tab.p ? tab.p + (k - 1) * per_sweep : nullptr;
     if (S.nsteps > 0) {
-      int nsteps = (int)S.nsteps;
-      unsigned stamp = (unsigned)k;
-      void *args[] = {&nsteps, &S.steps.p, &S.pos.p, &S.pred_ptr.p, &S.preds.p, &stamp,
-                      &done.p, &P.err.p, (void *)&budget, (void *)&stall, &a};
-      AIRT_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)k_kacz_dag, dim3(dag_grid),
+      const SweepArgs w{(int)S.nsteps, S.steps.p, S.ent.p, P.err.p, budget, stall};
+      if (k == 1) k_pack_pixels<<<grid_for(n, 256), 256, 0, s>>>((int)n, P.x64.p, xv.p);
+      void *args[] = {(void *)&w, &a};
+      AIRT_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)k_kacz_sweep, dim3(dag_grid),
                                                   dim3(kDagThreads), args, 0, s));
+      k_unpack_pixels<<<grid_for(n, 256), 256, 0, s>>>((int)n, P.x64.p, xv.p);
     }
     AIRT_LAUNCH_CHECK();
     AIRT_CHECK_CUDA(cudaMemcpyAsync(&herr, P.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));

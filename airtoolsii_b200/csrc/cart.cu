@@ -954,8 +954,11 @@ void run_cart(Problem &P, const airt_cart_opts &o, const double *d_b, const doub
     od.ensure(order.size());
     B = CartBlocks{plan.nblocks, plan.cbase.p, plan.ent.p, plan.gram.p, od.p};
     bsmem = 4 * kCartCols * kCartCols * sizeof(double) + (rsmem ? (size_t)m * sizeof(double) : 0);
+    // always the same limit: other threads may be launching
     AIRT_CHECK_CUDA(cudaFuncSetAttribute(rsmem ? k_cart_block<true> : k_cart_block<false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(4 * kCartCols * kCartCols * sizeof(double) +
+                                               kCartSharedRows * sizeof(double))));
     if (kmax >= o.kbegin) {  // some sweep may flag columns
       xold.ensure(n);
       tail.ensure(order.size());

@@ -172,13 +172,22 @@ struct SirtParams {
   int ncp_cols, ncp_smooth;
 };
 
-// Dependency schedule of a Kaczmarz row order (art.cu): the steps sorted by
-// level, their positions in the order, and each step's predecessors.
+// One step of a Kaczmarz schedule: its row, where the row's entries start in
+// the matrix and in the schedule's ranks, its position in the order, and the
+// entry of the row whose previous writer has the highest level (-1: none).
+struct ArtStep {
+  int64_t s0, off;
+  int len, row, pos, rep;
+};
+
+// Schedule of a Kaczmarz row order (art.cu): the steps sorted by level, and per
+// entry its pixel and how many earlier steps of the sweep write that pixel.
 struct ArtSchedule {
   int nlev = 0;
   int64_t nsteps = 0;
   uint64_t key = 0;  // hash of the row order it was built for (0: none)
-  DevBuf<int> steps, pos, pred_ptr, preds;
+  DevBuf<ArtStep> steps;
+  DevBuf<uint2> ent;
 };
 
 // Plan of the blocked CART sweep for a column order without repeats
