@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "ncp.cuh"
+#include "persist.cuh"
 #include "spmv.cuh"
 #include "trace.cuh"
 
@@ -78,6 +79,8 @@ struct Batch {
   DevBuf<uint16_t> ci16, ri16;
   DevBuf<double> rsq, nrm2, lam, taud, resn_last;
   bool tuned = false;
+  std::vector<int64_t> inst_nnz;  // nonzeros per instance (batch_tail), on first use
+  DevBuf<unsigned> tail_count;
   // active tiles per class, rebuilt after every stop-rule update:
   // tcount[c] row tiles, tcount[kClasses + c] column tiles of class c
   DevBuf<int> tcount;
@@ -514,6 +517,100 @@ __global__ void __launch_bounds__(256) k_batch_step(const int64_t *__restrict__ 
     stop[k] = 1;
     atomicSub(active, 1);
   }
+}
+
+// ---- the last instances of a solve in one launch
+// Once few instances run on, an iteration of the launched kernels is their
+// latency (seven kernels, 60-90 us, where a 64 x 64 instance moves 10 MB), so
+// the rest of the solve runs in one cooperative launch (persist.cuh): update,
+// residual and rule of all remaining instances, a grid barrier after each.
+constexpr int kTailInst = 32;          // instances at most
+constexpr int64_t kTailNnz = 16 << 20; // their nonzeros together at most
+constexpr int kTailThreads = 1024;
+
+struct TailArgs {
+  int count;                                 // instances
+  int inst[kTailInst];                       // their numbers
+  int prow[kTailInst + 1], pcol[kTailInst + 1];  // rows and columns before each
+  int64_t row0[kTailInst], col0[kTailInst];  // first row and column of each
+  PersistDir rows, cols;
+  BFwd f;
+  BUpd u;
+  BCtrl c;
+  int *stop, *iters, *rule;
+  double *resn;
+  unsigned *counter;
+  int *err;
+  long long budget;
+  int64_t kmax;
+};
+
+__global__ void __launch_bounds__(kTailThreads, 1) k_batch_tail(const __grid_constant__ TailArgs a, int n) {
+  __shared__ int live[kTailInst];
+  const int gt = blockIdx.x * kTailThreads + threadIdx.x, total = gridDim.x * kTailThreads;
+  const int lr = gt % a.rows.L, lc = gt % a.cols.L;
+  const int gr = gt / a.rows.L, gc = gt / a.cols.L, nr = total / a.rows.L, nc = total / a.cols.L;
+  const int R = a.prow[a.count], C = a.pcol[a.count];
+  unsigned target = 0;
+  auto barrier = [&]() {
+    return persist_barrier(a.counter, target += gridDim.x, a.err, a.budget, [] {});
+  };
+  // which instances run on; false when none does
+  auto look = [&]() -> bool {
+    int on = 0;
+    if (threadIdx.x < a.count) {
+      on = a.stop[a.inst[threadIdx.x]] == 0;
+      live[threadIdx.x] = on;
+    }
+    return __syncthreads_or(on) != 0;
+  };
+  if (!look()) return;
+  for (int it = 0; it < n; ++it) {
+    int x = 0;
+    for (int i = gc; !__all_sync(0xffffffffu, i >= C); i += nc) {
+      while (i < C && i >= a.pcol[x + 1]) ++x;
+      const bool on = i < C && live[x];
+      const int64_t j = on ? a.col0[x] + (i - a.pcol[x]) : a.cols.nseg;
+      const double g = persist_group_sum(persist_dot_again<2>(a.cols, (int)j, lc, a.f.mr32), a.cols.L);
+      if (on && lc == 0) {
+        double v = a.u.x64[j] + a.u.lam[a.inst[x]] * (a.u.D[j] * g);
+        if (a.u.lbk) v = fmax(v, a.u.lb);
+        if (a.u.ubk) v = fmin(v, a.u.ub);
+        a.u.x64[j] = v;
+        a.u.x32[j] = (float)v;
+      }
+    }
+    if (!barrier()) return;
+    x = 0;
+    for (int i = gr; !__all_sync(0xffffffffu, i >= R); i += nr) {
+      while (i < R && i >= a.prow[x + 1]) ++x;
+      const bool on = i < R && live[x];
+      const int64_t r = on ? a.row0[x] + (i - a.prow[x]) : a.rows.nseg;
+      const double s = persist_group_sum(persist_dot_again<2>(a.rows, (int)r, lr, a.u.x32), a.rows.L);
+      if (on && lr == 0) {
+        const double ri = a.f.b[r] - s;
+        a.f.mr32[r] = (float)(a.f.M[r] * ri);
+        a.f.rsq[r] = ri * ri;
+      }
+    }
+    if (!barrier()) return;
+    if (blockIdx.x < a.count && live[blockIdx.x]) {
+      const int k = a.inst[blockIdx.x];
+      const int64_t r0 = a.row0[blockIdx.x], m = a.prow[blockIdx.x + 1] - a.prow[blockIdx.x];
+      double v = 0.0;
+      for (int64_t i = threadIdx.x; i < m; i += kTailThreads) v += a.f.rsq[r0 + i];
+      v = block_sum<kTailThreads>(v);
+      if (threadIdx.x == 0 && batch_rule(k, 0, a.kmax, a.c, v, a.iters, a.rule, a.resn)) a.stop[k] = 1;
+    }
+    if (!barrier()) return;
+    if (!look()) return;
+  }
+}
+
+__global__ void k_pick_i64(int n, const int64_t *__restrict__ at, const int64_t *__restrict__ from,
+                           int64_t *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = from[at[i]];
 }
 
 __global__ void k_copy_f32(int64_t n, const double *__restrict__ a, float *__restrict__ b) {
@@ -1038,6 +1135,90 @@ void batch_ncp_setup(Batch &B) {
 }
 }  // namespace
 
+namespace {
+// Runs the instances that have not stopped to the end in one launch, when they
+// are few and small enough: the flags are read back (the stream is drained).
+// done: iterations every running instance has behind it.  Returns whether it
+// did.
+bool batch_tail(Batch &B, const BFwd &fo, const BUpd &uo, const BCtrl &co, int64_t done, int64_t kmax) {
+  Problem &P = B.P;
+  cudaStream_t s = P.stream;
+  const int K = B.ninst;
+  if (P.m >= INT32_MAX || P.n >= INT32_MAX) return false;
+  if (B.inst_nnz.empty()) {
+    DevBuf<int64_t> d;
+    d.ensure(K + 1);
+    k_pick_i64<<<(K + 256) / 256, 256, 0, s>>>(K + 1, B.d_row_off.p, P.rp.p, d.p);
+    AIRT_LAUNCH_CHECK();
+    std::vector<int64_t> h(K + 1);
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(h.data(), d.p, (K + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+    B.inst_nnz.resize(K);
+    for (int k = 0; k < K; ++k) B.inst_nnz[k] = h[k + 1] - h[k];
+  }
+  std::vector<int> hstop(K);
+  AIRT_CHECK_CUDA(cudaMemcpyAsync(hstop.data(), B.stop.p, K * sizeof(int), cudaMemcpyDeviceToHost, s));
+  AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+  TailArgs a{};
+  int64_t nnz = 0;
+  for (int k = 0; k < K; ++k) {
+    if (hstop[k]) continue;
+    if (a.count == kTailInst) return false;
+    const int64_t m = B.row_off[k + 1] - B.row_off[k], n = B.col_off[k + 1] - B.col_off[k];
+    const int q = a.count++;
+    nnz += B.inst_nnz[k];
+    if (nnz > kTailNnz || a.prow[q] + m >= INT32_MAX || a.pcol[q] + n >= INT32_MAX) return false;
+    a.inst[q] = k;
+    a.row0[q] = B.row_off[k];
+    a.col0[q] = B.col_off[k];
+    a.prow[q + 1] = a.prow[q] + (int)m;
+    a.pcol[q + 1] = a.pcol[q] + (int)n;
+  }
+  if (a.count == 0) return true;
+  const unsigned grid = (unsigned)num_sms();
+  if (a.count > (int)grid) return false;
+  int occ = 0;
+  AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_tail, kTailThreads, 0));
+  if (occ < 1) return false;
+  auto lanes = [&](int64_t nseg) {
+    return persist_lanes(nnz, nseg, (int64_t)grid * kTailThreads);
+  };
+  a.rows = PersistDir{(int)P.m, P.rp.p, P.ci.p, P.rv.p, lanes(a.prow[a.count])};
+  a.cols = PersistDir{(int)P.n, P.cp.p, P.ri.p, P.cv.p, lanes(a.pcol[a.count])};
+  a.f = fo;
+  a.u = uo;
+  a.c = co;
+  a.stop = B.stop.p;
+  a.iters = B.iters.p;
+  a.rule = B.rule.p;
+  a.resn = B.resn_last.p;
+  B.tail_count.ensure(1);
+  P.err.ensure(1);
+  AIRT_CHECK_CUDA(cudaMemsetAsync(P.err.p, 0, sizeof(int), s));
+  a.counter = B.tail_count.p;
+  a.err = P.err.p;
+  a.budget = g_persist_wait_budget;
+  a.kmax = kmax;
+  constexpr int64_t kIters = 2048;  // per launch
+  for (int64_t it = done; it < kmax;) {
+    int n = (int)std::min(kIters, kmax - it);
+    AIRT_CHECK_CUDA(cudaMemsetAsync(B.tail_count.p, 0, sizeof(unsigned), s));
+    void *args[] = {&a, &n};
+    AIRT_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)k_batch_tail, dim3(grid), dim3(kTailThreads), args,
+                                                0, s));
+    it += n;
+  }
+  int herr = 0;
+  AIRT_CHECK_CUDA(cudaMemcpyAsync(&herr, P.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+  if (herr) {
+    set_error("a bounded device wait of the batch's last instances gave up");
+    throw Status{AIRT_ERR_TIMEOUT};
+  }
+  return true;
+}
+}  // namespace
+
 // SIRT over the whole batch with per-instance relaxpar and a per-instance
 // stopping rule (rule: AIRT_STOP_NONE, DP, ME or NCP; taud_host per
 // instance for DP / ME; ncp_smooth values for NCP).
@@ -1136,8 +1317,19 @@ void batch_sirt(Batch &B, int method, const double *lam_host, const double *d_b,
   // queued (lagged poll), so the device never idles on the poll.
   const int64_t chunk = 8;
   const int lag = 2;
+  // rules whose last instances may finish in one launch, and the active count
+  // at which that was last tried in vain.  A solve of a few iterations is done
+  // before the flags would be back, and its first iterate stays the
+  // back projection bit for bit.
+  const bool tail_ok = !me && !ncp && kmax >= chunk;
+  int tried = K + 1;
+  bool finished = false;
+  if (tail_ok && K <= kTailInst) {
+    finished = batch_tail(B, fo, uo, co, 0, kmax);
+    tried = K;
+  }
   cudaGraphExec_t gexec = nullptr;
-  if (kmax >= chunk) {
+  if (kmax >= chunk && !finished) {
     cudaGraph_t g = nullptr;
     AIRT_CHECK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int64_t j = 0; j < chunk; ++j) iteration();
@@ -1153,7 +1345,7 @@ void batch_sirt(Batch &B, int method, const double *lam_host, const double *d_b,
   cudaEvent_t ev[3];
   for (int q = 0; q < 3; ++q) AIRT_CHECK_CUDA(cudaEventCreateWithFlags(&ev[q], cudaEventDisableTiming));
   int64_t c = 0;
-  for (int64_t it = 1; it <= kmax; ++c) {
+  for (int64_t it = 1; !finished && it <= kmax; ++c) {
     const int64_t cnt = std::min<int64_t>(chunk, kmax - it + 1);
     if (cnt == chunk && gexec) {
       AIRT_CHECK_CUDA(cudaGraphLaunch(gexec, s));
@@ -1167,7 +1359,12 @@ void batch_sirt(Batch &B, int method, const double *lam_host, const double *d_b,
     AIRT_CHECK_CUDA(cudaEventRecord(ev[c % 3], s));
     if (c >= lag) {
       AIRT_CHECK_CUDA(cudaEventSynchronize(ev[(c - lag) % 3]));
-      if (hact[(c - lag) % 3] == 0) break;
+      const int act = hact[(c - lag) % 3];
+      if (act == 0) break;
+      if (tail_ok && act <= kTailInst && act < tried && it <= kmax) {
+        finished = batch_tail(B, fo, uo, co, it - 1, kmax);
+        tried = act;
+      }
     }
   }
   for (int q = 0; q < 3; ++q) cudaEventDestroy(ev[q]);

@@ -35,6 +35,23 @@ struct PersistDir {
   int L;
 };
 
+// Lanes per segment for `threads` threads: the fewest vector loads in a row per
+// lane, where a segment's fixed part (bounds, reduction, epilogue) counts as
+// three.
+inline int persist_lanes(int64_t nnz, int64_t nseg, int64_t threads) {
+  const double avg = nseg ? (double)nnz / (double)nseg : 0.0;
+  int best = 2;
+  double cost = INFINITY;
+  for (int L = 2; L <= 32; L *= 2) {
+    const double c = std::ceil((double)nseg * L / (double)threads) * (avg / (4.0 * L) + 3.0);
+    if (c < cost) {
+      cost = c;
+      best = L;
+    }
+  }
+  return best;
+}
+
 // The resident part of a lane's first segment: vectors v, v + L, ... of the
 // aligned groups that overlap it, a mask bit per element inside the segment,
 // and where the rest of the segment's vectors starts.

@@ -803,21 +803,7 @@ void run_persist(Problem &P, const FwdOut &fo, const UpdArgs &ua, int64_t kmax) 
   cudaStream_t s = P.stream;
   auto kernel = k_sirt_persist<THREADS, R>;
   const unsigned grid = (unsigned)std::min(num_sms(), kPersistGrid);
-  // lanes per segment: the fewest vector loads in a row per lane, where a
-  // segment's fixed part (bounds, reduction, epilogue) counts as three
-  auto lanes = [&](int64_t nseg) {
-    const double avg = (double)P.nnz / (double)nseg;
-    int best = 2;
-    double cost = INFINITY;
-    for (int L = 2; L <= 32; L *= 2) {
-      const double c = std::ceil((double)nseg * L / ((double)grid * THREADS)) * (avg / (4.0 * L) + 3.0);
-      if (c < cost) {
-        cost = c;
-        best = L;
-      }
-    }
-    return best;
-  };
+  auto lanes = [&](int64_t nseg) { return persist_lanes(P.nnz, nseg, (int64_t)grid * THREADS); };
   int occ = 0;
   AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, 0));
   AIRT_REQUIRE(occ >= 1, "the one-launch SIRT kernel cannot be resident");
