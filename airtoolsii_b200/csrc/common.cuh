@@ -155,6 +155,7 @@ struct MultiState {
   int iter;    // global iteration whose residuals the control step judges next
   int active;  // instances not stopped
   double lam;  // relaxpar of the iteration being computed
+  int x_nonfinite, r_nonfinite;  // the FP32 copies of X, M.*R have held an infinity or NaN
 };
 
 struct SirtParams {

@@ -16,7 +16,7 @@
 //         gather (0 for stopped instances), per-block partial ||r_k||^2;
 //   ctrl: one block per instance sums the partials in a fixed order and
 //         applies check_stoprules.m's DP rule (or kmax) to that instance.
-// A lane owns 8 consecutive instances; a group of G lanes (G the smallest
+// A lane owns 8 instances (4 in each half of a row); a group of G lanes (G the smallest
 // power of two with 8G >= K, Kp = 8G slots, at most 256 per pass) walks one
 // row or column.  All sums
 // run in a fixed order, so results repeat bit for bit.  Matrix values and
@@ -48,48 +48,100 @@ struct MrArgs {
   const double *lamk;  // per-instance relaxpar [Kp], or null (st->lam for all)
 };
 
-__device__ __forceinline__ void load8(const float *p, float v[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-  const float4 b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+// Slot s = 0..7 of a lane: instances 4*lane + s of the row's first half and
+// 4*lane + s - 4 of its second half, so that the lanes of a group read each
+// half of a row of instances as consecutive 16-byte words.
+template <int G>
+__device__ __forceinline__ int slot_of(int lane, int s) {
+  return (s >> 2) * 4 * G + 4 * lane + (s & 3);
 }
 
+// The double that holds 2^-896 f for a finite f (exact, zeros and subnormal
+// floats included): the float's sign, exponent and fraction fields in the
+// double's places, the exponent not rebased.
+constexpr double kUnscale = 0x1p896;
+__device__ __forceinline__ double scaled_double(float f) {
+  const int b = __float_as_int(f);
+  return __hiloint2double((b >> 3) & (int)0x8fffffffu, b << 29);
+}
+constexpr int kXuSlots = 2;  // of each 4 slots: the ones widened by the conversion unit
+
 // Walk segment i (row of the CSR or column of the CSC) with a group of G
-// lanes: acc[s] = sum_q val[q] * vec[idx[q]][8*lane + s].
-template <int G>
+// lanes: acc[s] = sum_q val[q] * vec[idx[q]][slot_of(lane, s)], in the order
+// of the nonzeros.  The 16-byte aligned groups of four nonzeros that overlap
+// the segment are read whole, the next group's values and indices while the
+// current one's gathers are in flight; nonzeros of the neighbouring segments
+// count with the value 0 and gather a row of the segment itself.
+//
+// Bound by the conversions: every FP32 operand has to be widened for the
+// FP64 FMA, and the conversion unit takes 16 lanes per cycle and SM.  FINITE:
+// part of the operands are widened by integer instructions, times 2^-896,
+// against a value times 2^896 - the products are exact, so every FMA rounds
+// as with the plain operands.  An infinity or NaN would not survive that:
+// the kernel that writes vec notes any (MultiState), and FINITE is off.
+//
+// N = 256, 60 angles, 256 slots: 0.54 ms per direction with every operand
+// through the conversion unit (66 % busy) and 8 consecutive instances per
+// lane (half of each 32-byte sector pair per load), 0.40 ms now (conversion
+// 50 %, issue 52 %, L1 54-61 %).  kXuSlots 0, 1, 2 of 4: 20.3, 19.5, 19.6 ms
+// for 250 warm-started solves; three blocks per SM spill, 20.7 ms.
+template <int G, bool FINITE>
 __device__ __forceinline__ void seg_dot(int64_t q0, int64_t q1, const int *__restrict__ idx,
                                         const float *__restrict__ val,
-                                        const float *__restrict__ vec, int Kp, int lane,
-                                        double acc[8]) {
+                                        const float *__restrict__ vec, int lane,
+                                        double (&acc)[8]) {
 #pragma unroll
   for (int s = 0; s < 8; ++s) acc[s] = 0.0;
-  int64_t q = q0;
-  // four nonzeros per round: their indices, values and gathers are all in
-  // flight before the first FMA; the FMAs run in nonzero order
-  for (; q + 4 <= q1; q += 4) {
-    int c[4];
-    float v[4];
+  if (q0 >= q1) return;
+  const float *base = vec + 4 * lane;
+  int64_t w = q0 >> 2;
+  const int64_t we = (q1 + 3) >> 2;
+  int4 c4 = __ldg(reinterpret_cast<const int4 *>(idx) + w);
+  float4 v4 = __ldg(reinterpret_cast<const float4 *>(val) + w);
+  for (; w < we; ++w) {
+    int c[4] = {c4.x, c4.y, c4.z, c4.w};
+    float v[4] = {v4.x, v4.y, v4.z, v4.w};
+    const int lo = q0 > 4 * w ? (int)(q0 - 4 * w) : 0;
+    const int hi = q1 < 4 * w + 4 ? (int)(q1 - 4 * w) : 4;
+    if (hi - lo < 4) {
+      const int own = lo == 0 ? c[0] : lo == 1 ? c[1] : lo == 2 ? c[2] : c[3];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (u < lo || u >= hi) {
+          c[u] = own;
+          v[u] = 0.0f;
+        }
+    }
+    float4 g[4][2];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      c[u] = __ldg(idx + q + u);
-      v[u] = __ldg(val + q + u);
+      const float4 *p = reinterpret_cast<const float4 *>(base + (int64_t)c[u] * (8 * G));
+      g[u][0] = __ldg(p);
+      g[u][1] = __ldg(p + G);
     }
-    float g[4][8];
+    if (w + 1 < we) {
+      c4 = __ldg(reinterpret_cast<const int4 *>(idx) + w + 1);
+      v4 = __ldg(reinterpret_cast<const float4 *>(val) + w + 1);
+    }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) load8(vec + (int64_t)c[u] * Kp + 8 * lane, g[u]);
+    for (int u = 0; u < 4; ++u) {
+      const double a = (double)v[u], as = a * kUnscale;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+      for (int h = 0; h < 2; ++h) {
+        const float x[4] = {g[u][h].x, g[u][h].y, g[u][h].z, g[u][h].w};
 #pragma unroll
-      for (int s = 0; s < 8; ++s) acc[s] = fma((double)v[u], (double)g[u][s], acc[s]);
-  }
-  for (; q < q1; ++q) {
-    const int c = __ldg(idx + q);
-    const double v = (double)__ldg(val + q);
-    float g[8];
-    load8(vec + (int64_t)c * Kp + 8 * lane, g);
-#pragma unroll
-    for (int s = 0; s < 8; ++s) acc[s] = fma(v, (double)g[s], acc[s]);
+        for (int s = 0; s < 4; ++s) {
+          double &t = acc[4 * h + s];
+          if (!FINITE) {
+            if (u >= lo && u < hi) t = fma(a, (double)x[s], t);
+          } else if (s < kXuSlots) {
+            t = fma(a, (double)x[s], t);
+          } else {
+            t = fma(as, scaled_double(x[s]), t);
+          }
+        }
+      }
+    }
   }
 }
 
@@ -104,7 +156,7 @@ __device__ __forceinline__ void block_partials(double part[8], double *__restric
     for (int o = G; o < 32; o <<= 1) part[s] += __shfl_xor_sync(0xffffffffu, part[s], o);
   if (lane32 < G)
 #pragma unroll
-    for (int s = 0; s < 8; ++s) sh[warp][8 * lane32 + s] = part[s];
+    for (int s = 0; s < 8; ++s) sh[warp][slot_of<G>(lane32, s)] = part[s];
   __syncthreads();
   for (int k = threadIdx.x; k < Kp; k += blockDim.x) {
     double a = 0.0;
@@ -114,71 +166,106 @@ __device__ __forceinline__ void block_partials(double part[8], double *__restric
 }
 
 // R = B - A*X, M.*R (FP32, 0 for stopped instances), per-block ||r_k||^2.
+template <int G, bool FINITE>
+__device__ __forceinline__ void mr_fwd_rows(int64_t m, const int64_t *__restrict__ rp,
+                                            const int *__restrict__ ci,
+                                            const float *__restrict__ rv, const MrArgs &a,
+                                            double (&part)[8]) {
+  const int lane = threadIdx.x % G;
+  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+  const int64_t ng = (int64_t)gridDim.x * blockDim.x / G;
+  constexpr int Kp = 8 * G;
+  bool live[8];
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    const int k = slot_of<G>(lane, s);
+    live[s] = k < a.K && !a.stop[k];
+  }
+  bool finite = true;
+  for (int64_t i = gid; i < m; i += ng) {
+    double acc[8];
+    seg_dot<G, FINITE>(__ldg(rp + i), __ldg(rp + i + 1), ci, rv, a.x32, lane, acc);
+    const double Mi = __ldg(a.M + i);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t at = i * Kp + slot_of<G>(lane, 4 * h);
+      const double2 b0 = __ldg(reinterpret_cast<const double2 *>(a.bil + at));
+      const double2 b1 = __ldg(reinterpret_cast<const double2 *>(a.bil + at) + 1);
+      const double bi[4] = {b0.x, b0.y, b1.x, b1.y};
+      float mr[4];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const double r = bi[s] - acc[4 * h + s];
+        const bool on = live[4 * h + s];
+        mr[s] = on ? (float)(Mi * r) : 0.0f;
+        part[4 * h + s] += on ? r * r : 0.0;
+        finite = finite && isfinite(mr[s]);
+      }
+      *reinterpret_cast<float4 *>(a.mr32 + at) = make_float4(mr[0], mr[1], mr[2], mr[3]);
+    }
+  }
+  if (!finite) a.st->r_nonfinite = 1;
+}
+
 template <int G>
 __global__ void __launch_bounds__(kMrThreads, 2) k_mr_fwd(int64_t m, const int64_t *__restrict__ rp,
                                                        const int *__restrict__ ci,
                                                        const float *__restrict__ rv, MrArgs a) {
   if (a.st->active == 0) return;
-  const int lane = threadIdx.x % G;
-  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
-  const int64_t ng = (int64_t)gridDim.x * blockDim.x / G;
-  const int Kp = a.Kp;
-  bool live[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) live[s] = (8 * lane + s) < a.K && !a.stop[8 * lane + s];
   double part[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int64_t i = gid; i < m; i += ng) {
-    double acc[8];
-    seg_dot<G>(__ldg(rp + i), __ldg(rp + i + 1), ci, rv, a.x32, Kp, lane, acc);
-    const double Mi = __ldg(a.M + i);
-    const double *bi = a.bil + i * Kp + 8 * lane;
-    float mr[8];
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const double r = __ldg(bi + s) - acc[s];
-      mr[s] = live[s] ? (float)(Mi * r) : 0.0f;
-      part[s] += live[s] ? r * r : 0.0;
-    }
-    float4 *o = reinterpret_cast<float4 *>(a.mr32 + i * Kp + 8 * lane);
-    o[0] = make_float4(mr[0], mr[1], mr[2], mr[3]);
-    o[1] = make_float4(mr[4], mr[5], mr[6], mr[7]);
-  }
-  block_partials<G>(part, a.partial, Kp);
+  if (a.st->x_nonfinite)
+    mr_fwd_rows<G, false>(m, rp, ci, rv, a, part);
+  else
+    mr_fwd_rows<G, true>(m, rp, ci, rv, a, part);
+  block_partials<G>(part, a.partial, a.Kp);
 }
 
 // g = A'*(M.*R); x += lam*D.*g, box projection, FP32 copy (running instances).
+template <int G, bool FINITE>
+__device__ __forceinline__ void mr_bwd_cols(int64_t n, const int64_t *__restrict__ cp,
+                                            const int *__restrict__ ri,
+                                            const float *__restrict__ cv, const MrArgs &a) {
+  const int lane = threadIdx.x % G;
+  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+  const int64_t ng = (int64_t)gridDim.x * blockDim.x / G;
+  constexpr int Kp = 8 * G;
+  double lam[8];
+  bool live[8];
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    const int k = slot_of<G>(lane, s);
+    live[s] = k < a.K && !a.stop[k];
+    lam[s] = a.lamk ? a.lamk[k] : a.st->lam;
+  }
+  bool finite = true;
+  for (int64_t j = gid; j < n; j += ng) {
+    double g[8];
+    seg_dot<G, FINITE>(__ldg(cp + j), __ldg(cp + j + 1), ri, cv, a.mr32, lane, g);
+    const double Dj = __ldg(a.D + j);
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      if (!live[s]) continue;
+      const int64_t at = j * Kp + slot_of<G>(lane, s);
+      double x = a.x64[at] + lam[s] * (Dj * g[s]);
+      if (a.lbk) x = fmax(x, a.lb);
+      if (a.ubk) x = fmin(x, a.ub);
+      a.x64[at] = x;
+      a.x32[at] = (float)x;
+      finite = finite && isfinite((float)x);
+    }
+  }
+  if (!finite) a.st->x_nonfinite = 1;
+}
+
 template <int G>
 __global__ void __launch_bounds__(kMrThreads, 2) k_mr_bwd(int64_t n, const int64_t *__restrict__ cp,
                                                        const int *__restrict__ ri,
                                                        const float *__restrict__ cv, MrArgs a) {
   if (a.st->active == 0) return;
-  const int lane = threadIdx.x % G;
-  const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
-  const int64_t ng = (int64_t)gridDim.x * blockDim.x / G;
-  const int Kp = a.Kp;
-  double lam[8];
-  bool live[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    live[s] = (8 * lane + s) < a.K && !a.stop[8 * lane + s];
-    lam[s] = a.lamk ? a.lamk[8 * lane + s] : a.st->lam;
-  }
-  for (int64_t j = gid; j < n; j += ng) {
-    double g[8];
-    seg_dot<G>(__ldg(cp + j), __ldg(cp + j + 1), ri, cv, a.mr32, Kp, lane, g);
-    const double Dj = __ldg(a.D + j);
-    double *xj = a.x64 + j * Kp + 8 * lane;
-    float *xj32 = a.x32 + j * Kp + 8 * lane;
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      if (!live[s]) continue;
-      double x = xj[s] + lam[s] * (Dj * g[s]);
-      if (a.lbk) x = fmax(x, a.lb);
-      if (a.ubk) x = fmin(x, a.ub);
-      xj[s] = x;
-      xj32[s] = (float)x;
-    }
-  }
+  if (a.st->r_nonfinite)
+    mr_bwd_cols<G, false>(n, cp, ri, cv, a);
+  else
+    mr_bwd_cols<G, true>(n, cp, ri, cv, a);
 }
 
 // One block per instance: ||r_k||^2 from the per-block partials (fixed
@@ -217,7 +304,8 @@ __global__ void k_mr_advance(MultiState *st, const double *relax_table, double r
 
 // [K][len] instance-major <-> [len][Kp] interleaved, through 32 x 32 tiles.
 __global__ void k_to_interleaved(int64_t len, int K, int Kp, const double *__restrict__ src,
-                                 double *__restrict__ dst, float *__restrict__ dst32) {
+                                 double *__restrict__ dst, float *__restrict__ dst32,
+                                 int *__restrict__ nonfinite) {
   __shared__ double t[32][33];
   const int64_t i0 = (int64_t)blockIdx.x * 32;
   const int k0 = blockIdx.y * 32;
@@ -233,7 +321,10 @@ __global__ void k_to_interleaved(int64_t len, int K, int Kp, const double *__res
     if (i < len && k < Kp) {
       const double v = t[threadIdx.x][r];
       dst[i * Kp + k] = v;
-      if (dst32) dst32[i * Kp + k] = (float)v;
+      if (dst32) {
+        dst32[i * Kp + k] = (float)v;
+        if (!isfinite((float)v)) *nonfinite = 1;
+      }
     }
   }
 }
@@ -333,11 +424,14 @@ void multi_pass(Problem &P, const airt_sirt_opts &o, int K0, const double *d_B, 
   P.mr_x64.ensure((size_t)n * Kp);
   P.mr_x32.ensure((size_t)n * Kp);
   P.mr_r32.ensure((size_t)m * Kp);
+  MultiState st0{0, K, o.relaxpar, 0, 0};
+  P.mr_state.ensure(1);
+  P.mr_state.upload(&st0, 1, s);
   const dim3 tb(32, 8);
   k_to_interleaved<<<dim3((unsigned)((m + 31) / 32), (unsigned)((Kp + 31) / 32)), tb, 0, s>>>(
-      m, K, Kp, d_B, P.mr_b.p, nullptr);
+      m, K, Kp, d_B, P.mr_b.p, nullptr, nullptr);
   k_to_interleaved<<<dim3((unsigned)((n + 31) / 32), (unsigned)((Kp + 31) / 32)), tb, 0, s>>>(
-      n, K, Kp, d_X0, P.mr_x64.p, P.mr_x32.p);
+      n, K, Kp, d_X0, P.mr_x64.p, P.mr_x32.p, &P.mr_state.p->x_nonfinite);
   AIRT_LAUNCH_CHECK();
   auto grids = [&](unsigned &gf, unsigned &gb) {
     gf = std::min<unsigned>(grid_for(m * G, kMrThreads, 8), (unsigned)num_sms() * 8);
@@ -350,12 +444,9 @@ void multi_pass(Problem &P, const airt_sirt_opts &o, int K0, const double *d_B, 
   P.mr_iters.ensure(Kp);
   P.mr_rule.ensure(Kp);
   P.mr_resn.ensure(Kp);
-  P.mr_state.ensure(1);
   AIRT_CHECK_CUDA(cudaMemsetAsync(P.mr_stop.p, 0, Kp * sizeof(int), s));
   AIRT_CHECK_CUDA(cudaMemsetAsync(P.mr_iters.p, 0, Kp * sizeof(int), s));
   AIRT_CHECK_CUDA(cudaMemsetAsync(P.mr_rule.p, 0, Kp * sizeof(int), s));
-  MultiState st0{0, K, o.relaxpar};
-  P.mr_state.upload(&st0, 1, s);
   // per-slot copies of the per-instance inputs (slot q holds instance orig[q])
   std::vector<int> orig(K);
   for (int k = 0; k < K; ++k) orig[k] = k;
