@@ -286,13 +286,13 @@ void conv3x3_bf16(const GemmArgs &g0, int bn, int epi, cudaStream_t s) {
   AIRT_REQUIRE(((uintptr_t)g.convX & 15) == 0 && ((uintptr_t)g.B & 15) == 0 && g.ldb % 8 == 0,
                "conv3x3: operands must be 16-byte aligned");
   AIRT_REQUIRE(g.K % BK == 0, "conv3x3: K must be padded to a multiple of 64");
-  AIRT_REQUIRE(epi == EPI_BIAS_RELU_BF16 || epi == EPI_BIAS_BF16 || epi == EPI_ADD_F32,
+  AIRT_REQUIRE(epi == EPI_BIAS_RELU_BF16 || epi == EPI_BIAS_BF16 || epi == EPI_STORE_F32,
                "conv3x3: unsupported epilogue");
   g.ksplit = g.K;
 #define AIRT_C(BNV)                                                                     \
   if (epi == EPI_BIAS_RELU_BF16) launch<BNV, false, false, EPI_BIAS_RELU_BF16, 1>(g, s); \
   else if (epi == EPI_BIAS_BF16) launch<BNV, false, false, EPI_BIAS_BF16, 1>(g, s);      \
-  else launch<BNV, false, false, EPI_ADD_F32, 1>(g, s);
+  else launch<BNV, false, false, EPI_STORE_F32, 1>(g, s);
   switch (bn) {
     case 32: AIRT_C(32) break;
     case 64: AIRT_C(64) break;

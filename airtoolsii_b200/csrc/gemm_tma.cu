@@ -944,7 +944,6 @@ void dispatch_tma(const CUtensorMap &ma, const CUtensorMap &mb, const GemmArgs &
     case EPI_STORE_F32: launch_tma<BNV, EPI_STORE_F32, MODE, SWA, SWB>(ma, mb, g, geo, s); break;       \
     case EPI_BIAS_RELU_BF16: launch_tma<BNV, EPI_BIAS_RELU_BF16, MODE, SWA, SWB>(ma, mb, g, geo, s); break; \
     case EPI_BIAS_BF16: launch_tma<BNV, EPI_BIAS_BF16, MODE, SWA, SWB>(ma, mb, g, geo, s); break;       \
-    case EPI_ADD_F32: launch_tma<BNV, EPI_ADD_F32, MODE, SWA, SWB>(ma, mb, g, geo, s); break;           \
     default: launch_tma<BNV, EPI_ATOMIC_F32_T, MODE, SWA, SWB>(ma, mb, g, geo, s); break;               \
   }
   switch (bn) {
@@ -1106,7 +1105,6 @@ static bool conv3x3_rows(const GemmArgs &g, int bn, int epi, cudaStream_t s) {
       launch_rows<BNV, EPI_BIAS_RELU_BF16, SWV, ONEV>(ma, mb, g, geo, smem, grid, s);                     \
       break;                                                                                              \
     case EPI_BIAS_BF16: launch_rows<BNV, EPI_BIAS_BF16, SWV, ONEV>(ma, mb, g, geo, smem, grid, s); break; \
-    case EPI_ADD_F32: launch_rows<BNV, EPI_ADD_F32, SWV, ONEV>(ma, mb, g, geo, smem, grid, s); break;     \
     default: return false;                                                                                \
   }
   if (sw == 128) {
@@ -1211,7 +1209,6 @@ static bool conv3x3_stack(const GemmArgs &g, int bn, int epi, cudaStream_t s) {
       launch_stack<BNV, EPI_BIAS_RELU_BF16, SWV, ONEV>(ma, mb, md, g, geo, smem, grid, s);                \
       break;                                                                                              \
     case EPI_BIAS_BF16: launch_stack<BNV, EPI_BIAS_BF16, SWV, ONEV>(ma, mb, md, g, geo, smem, grid, s); break; \
-    case EPI_ADD_F32: launch_stack<BNV, EPI_ADD_F32, SWV, ONEV>(ma, mb, md, g, geo, smem, grid, s); break; \
     default: return false;                                                                                \
   }
   if (sw == 128) {

@@ -150,7 +150,6 @@ enum GemmEpi {
   EPI_BIAS_RELU_BF16 = 1, // relu(D + bias[n]) -> bf16 [M][ldd]
   EPI_BIAS_BF16 = 2,      // D + bias[n] -> bf16
   EPI_ATOMIC_F32_T = 3,   // atomicAdd(D) into fp32 stored transposed [N][ldd] (split-K)
-  EPI_ADD_F32 = 4,        // D += result, fp32 [M][ldd] (no split-K)
 };
 
 struct GemmArgs {
@@ -194,20 +193,8 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs &g, uint32_t taddr,
     }
     const int col0 = n0 + c;
     if (EPI != EPI_ATOMIC_F32_T && vec_ok && row < g.M && col0 + 32 <= g.N) {
-      if (EPI == EPI_STORE_F32 || EPI == EPI_ADD_F32) {
+      if (EPI == EPI_STORE_F32) {
         float4 *d = reinterpret_cast<float4 *>((float *)g.D + (size_t)row * g.ldd + col0);
-        if (EPI == EPI_ADD_F32) {
-          float4 o[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = d[j];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            v[4 * j] += o[j].x;
-            v[4 * j + 1] += o[j].y;
-            v[4 * j + 2] += o[j].z;
-            v[4 * j + 3] += o[j].w;
-          }
-        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) d[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
       } else {
@@ -253,8 +240,6 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs &g, uint32_t taddr,
           y += g.bias ? g.bias[col] : 0.f;
           if (EPI == EPI_BIAS_RELU_BF16) y = fmaxf(y, 0.f);
           ((__nv_bfloat16 *)g.D)[(size_t)row * g.ldd + col] = __float2bfloat16(y);
-        } else if (EPI == EPI_ADD_F32) {
-          ((float *)g.D)[(size_t)row * g.ldd + col] += y;
         } else {
           atomicAdd((float *)g.D + (size_t)col * g.ldd + row, y);
         }
