@@ -1197,7 +1197,7 @@ bool batch_tail(Batch &B, const BFwd &fo, const BUpd &uo, const BCtrl &co, int64
   AIRT_CHECK_CUDA(cudaMemsetAsync(P.err.p, 0, sizeof(int), s));
   a.counter = B.tail_count.p;
   a.err = P.err.p;
-  a.budget = g_persist_wait_budget;
+  a.budget = kPersistWaitBudget;
   a.kmax = kmax;
   constexpr int64_t kIters = 2048;  // per launch
   for (int64_t it = done; it < kmax;) {

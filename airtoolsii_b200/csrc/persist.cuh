@@ -22,8 +22,8 @@
 
 namespace airt {
 
-// Test hook: cycle budget of a barrier wait (~2 s).
-inline long long g_persist_wait_budget = 4000000000ll;
+// Cycle budget of a barrier wait (~2 s).
+constexpr long long kPersistWaitBudget = 4000000000ll;
 
 // One direction of the matrix: segments ptr[i]..ptr[i+1] of idx and val, L
 // lanes per segment.

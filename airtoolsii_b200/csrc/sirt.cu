@@ -820,7 +820,7 @@ void run_persist(Problem &P, const FwdOut &fo, const UpdArgs &ua, int64_t kmax) 
   a.part = P.pst_part.p;
   a.count = P.pst_count.p;
   a.err = P.err.p;
-  a.budget = g_persist_wait_budget;
+  a.budget = kPersistWaitBudget;
   ensure_h_state(P);
   for (int64_t it = 0; it < kmax; it = a.it1) {
     a.it0 = (int)it;

@@ -7,13 +7,15 @@
 //    stable transposition.  Row entries keep the ray order of the trace.
 //    Replaces testprobs/paralleltomo.m:112-301, fanlineartomo.m:141-358 and
 //    seismictomo.m:96-287 (isMatrix = 1).
-//  * apply_matrix_free: forward projection (one thread per ray, FP64 sum in
-//    ray order) and back projection (one thread per ray, scatter in 64-bit
-//    fixed point, so the result does not depend on the order in which rays
-//    arrive) that re-trace every ray, as the isMatrix = 0 handles of
-//    paralleltomo.m:280-288 do.  Entry values are rounded to FP32 exactly as
-//    the stored matrix holds them, so stored and matrix-free operators agree
-//    up to summation order.
+//  * apply_matrix_free: forward projection (the grid walk of dda.cuh, a ray
+//    in parts of 4 or 8 threads) and back projection (parallel beams: a gather
+//    per pixel, gather.cuh; the others: a scatter in 64-bit fixed point, so
+//    the result does not depend on the order in which rays arrive), as the
+//    isMatrix = 0 handles of paralleltomo.m:280-288 do.  Entry values are
+//    rounded to FP32 as the stored matrix holds them; where a length lies at a
+//    rounding boundary (about one entry in a million) the two differ by one
+//    FP32 unit in the last place.  sphericaltomo and rays the walk refuses are
+//    traced by the tracer of trace.cuh.
 #include <climits>
 #include <cstring>
 
