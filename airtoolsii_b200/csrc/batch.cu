@@ -55,9 +55,17 @@ constexpr int kClasses = 5;
 struct TileSet {
   int ntiles = 0;
   DevBuf<int> cls, list;
+  std::vector<int> hcls;  // cls on the host
   int count[kClasses] = {};
   int off[kClasses] = {};
   int lanes[kClasses] = {2, 4, 4, 8, 8};
+};
+
+// Consecutive segments of one of the last instances (k_batch_tail) whose tiles
+// have the same class; pieces are sorted by class, `start` counts the class's
+// segments before it, `slot` the instance among the last ones.
+struct TailPiece {
+  int first, count, start, slot;
 };
 
 struct ClassOffsets {
@@ -81,6 +89,7 @@ struct Batch {
   bool tuned = false;
   std::vector<int64_t> inst_nnz;  // nonzeros per instance (batch_tail), on first use
   DevBuf<unsigned> tail_count;
+  DevBuf<TailPiece> tail_pr, tail_pc;  // rows and columns of the last instances
   // active tiles per class, rebuilt after every stop-rule update:
   // tcount[c] row tiles, tcount[kClasses + c] column tiles of class c
   DevBuf<int> tcount;
@@ -221,6 +230,14 @@ struct BFwd {
   double *ppr;
 };
 
+// r = b - (A*x) of a row, M.*r and r.^2; returns r.
+__device__ __forceinline__ double batch_residual(int64_t row, double s, double b, double M, const BFwd &o) {
+  const double r = b - s;
+  o.mr32[row] = (float)(M * r);
+  o.rsq[row] = r * r;
+  return r;
+}
+
 // Residual pass; with idx16 (16-bit local column indices, voff = the
 // instances' first columns) the nonzeros stream at 6 bytes instead of 8.
 template <int L>
@@ -233,9 +250,7 @@ __global__ void __launch_bounds__(256, kBatchCtas)
   auto epi = [&](int64_t i, double s, bool lead, double2 bm) {
         if (!lead) return;
         const int64_t r = o.r0 + i;
-        const double ri = bm.x - s;
-        o.mr32[r] = (float)(bm.y * ri);
-        o.rsq[r] = ri * ri;
+        const double ri = batch_residual(r, s, bm.x, bm.y, o);
         if (o.rprev) {
           if (o.pp) {
             const double pv = o.rprev[r];
@@ -264,6 +279,15 @@ struct BUpd {
   int64_t c0;
 };
 
+// x(c) from its old value, lambda, D(c) and the column's sum g.
+__device__ __forceinline__ void batch_update(int64_t c, double g, double x0, double lam, double D, const BUpd &u) {
+  double x = x0 + lam * (D * g);
+  if (u.lbk) x = fmax(x, u.lb);
+  if (u.ubk) x = fmin(x, u.ub);
+  u.x64[c] = x;
+  u.x32[c] = (float)x;
+}
+
 // Update pass; idx16 / voff as in k_batch_fwd (16-bit local row indices,
 // the instances' first rows).
 template <int L>
@@ -277,13 +301,7 @@ __global__ void __launch_bounds__(256, kBatchCtas)
     return make_double3(u.x64[c], u.lam[u.inst_col[c]], u.D[c]);
   };
   auto epi = [&](int64_t j, double g, bool lead, double3 xld) {
-        if (!lead) return;
-        const int64_t c = u.c0 + j;
-        double x = xld.x + xld.y * (xld.z * g);
-        if (u.lbk) x = fmax(x, u.lb);
-        if (u.ubk) x = fmin(x, u.ub);
-        u.x64[c] = x;
-        u.x32[c] = (float)x;
+        if (lead) batch_update(u.c0 + j, g, xld.x, xld.y, xld.z, u);
       };
   if (idx16)
     for_each_segment_vt16<L>(nseg, tiles, ntiles, kTileShift, cp + u.c0, idx16, cv, mr32, u.inst_col + u.c0, u.stop,
@@ -521,19 +539,45 @@ __global__ void __launch_bounds__(256) k_batch_step(const int64_t *__restrict__ 
 
 // ---- the last instances of a solve in one launch
 // Once few instances run on, an iteration of the launched kernels is their
-// latency (seven kernels, 60-90 us, where a 64 x 64 instance moves 10 MB), so
-// the rest of the solve runs in one cooperative launch (persist.cuh): update,
-// residual and rule of all remaining instances, a grid barrier after each.
-constexpr int kTailInst = 32;          // instances at most
+// latency (seven kernels, 60-90 us in a batch of many sizes, where a 64 x 64
+// instance moves 10 MB), so the rest of the solve runs in one cooperative
+// launch (persist.cuh): update, residual and rule of all remaining instances,
+// a grid barrier after each.
+//
+// Every sum is taken in the order of the launched kernels - a segment with
+// the lanes, indices and accumulators of its tile's class, a norm over 256
+// threads - so an instance's iterates do not depend on where its solve
+// finished.  (An FP64 sum in another order differs in its last bit, which
+// flips the FP32 rounding of x or M.*r now and then: up to 1e-8 of x after
+// hundreds of iterations.)
+//
+// us per iteration, one launch / launched kernels, in batches that hold these
+// instances alone: 0.31 M nonzeros 13.7 / 16.0, 1.9 M 20.8 / 25.1, 5 M 38 / 39,
+// 10 M 61 / 67, 15 M 78-90 / 85-96, 20 M 110 / 110, 30 M 144 / 148.  The two
+// meet at 15-20 M; kTailNnz lies there.
+constexpr int kTailInst = 32;          // instances at most (what the arguments hold)
 constexpr int64_t kTailNnz = 16 << 20; // their nonzeros together at most
 constexpr int kTailThreads = 1024;
+constexpr int kTailPieces = 256;       // pieces per direction at most
+
+struct TailDir {
+  const int64_t *ptr;
+  const int *idx;
+  const uint16_t *idx16;  // of the classes that read 16-bit indices, or null
+  const float *val;
+  const TailPiece *pieces;
+  int p0[kClasses + 1];  // first piece of every class
+  int total[kClasses];   // segments of every class
+  int shift[kClasses];   // thread that takes a class's first segment
+  int lanes[kClasses];
+};
 
 struct TailArgs {
-  int count;                                 // instances
-  int inst[kTailInst];                       // their numbers
-  int prow[kTailInst + 1], pcol[kTailInst + 1];  // rows and columns before each
+  int count;                // instances
+  int inst[kTailInst];      // their numbers
   int64_t row0[kTailInst], col0[kTailInst];  // first row and column of each
-  PersistDir rows, cols;
+  int m[kTailInst];         // rows of each
+  TailDir rows, cols;
   BFwd f;
   BUpd u;
   BCtrl c;
@@ -545,12 +589,57 @@ struct TailArgs {
   int64_t kmax;
 };
 
+// Every segment of class c that belongs to a running instance: epi(i, slot,
+// sum) on the first lane of its group of L.  voff: where the vector of a
+// slot's instance starts (W16).
+template <int L, bool W16, class Epi>
+__device__ __forceinline__ void tail_class(const TailDir &d, const TailPiece *pieces, int c, const int *live,
+                                           const int64_t *voff, const float *x, Epi &&epi) {
+  const int threads = gridDim.x * kTailThreads;
+  int t = blockIdx.x * kTailThreads + threadIdx.x - d.shift[c];
+  if (t < 0) t += threads;
+  const int lane = t % L, groups = threads / L, n = d.total[c];
+  const TailPiece *p = pieces + d.p0[c];
+  for (int i = t / L; !__all_sync(0xffffffffu, i >= n); i += groups) {
+    while (i < n && i >= p->start + p->count) ++p;
+    const bool on = i < n && live[p->slot];
+    const int seg = p->first + (i - p->start);
+    double s = 0.0;
+    if (on) {
+      const int64_t q0 = __ldg(d.ptr + seg), q1 = __ldg(d.ptr + seg + 1);
+      if (W16) s = segment_part16<L, true>(q0, q1, lane, d.idx16, d.val, x + voff[p->slot]);
+      else s = segment_part<L, true>(q0, q1, lane, d.idx, d.val, x);
+    }
+    s = group_sum<L>(s);
+    if (on && lane == 0) epi(seg, p->slot, s);
+  }
+}
+
+template <class Epi>
+__device__ __forceinline__ void tail_pass(const TailDir &d, const TailPiece *pieces, const int *live,
+                                          const int64_t *voff, const float *x, Epi &&epi) {
+#pragma unroll 1
+  for (int c = 0; c < kClasses; ++c) {
+    if (!d.total[c]) continue;
+    const bool w16 = d.idx16 && c >= kClasses - 2;
+    switch (d.lanes[c] + w16) {
+      case 2: tail_class<2, false>(d, pieces, c, live, voff, x, epi); break;
+      case 3: tail_class<2, true>(d, pieces, c, live, voff, x, epi); break;
+      case 4: tail_class<4, false>(d, pieces, c, live, voff, x, epi); break;
+      case 5: tail_class<4, true>(d, pieces, c, live, voff, x, epi); break;
+      case 8: tail_class<8, false>(d, pieces, c, live, voff, x, epi); break;
+      case 9: tail_class<8, true>(d, pieces, c, live, voff, x, epi); break;
+      case 16: tail_class<16, false>(d, pieces, c, live, voff, x, epi); break;
+      default: tail_class<16, true>(d, pieces, c, live, voff, x, epi); break;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kTailThreads, 1) k_batch_tail(const __grid_constant__ TailArgs a, int n) {
   __shared__ int live[kTailInst];
-  const int gt = blockIdx.x * kTailThreads + threadIdx.x, total = gridDim.x * kTailThreads;
-  const int lr = gt % a.rows.L, lc = gt % a.cols.L;
-  const int gr = gt / a.rows.L, gc = gt / a.cols.L, nr = total / a.rows.L, nc = total / a.cols.L;
-  const int R = a.prow[a.count], C = a.pcol[a.count];
+  __shared__ TailPiece pr[kTailPieces], pc[kTailPieces];
+  for (int q = threadIdx.x; q < a.rows.p0[kClasses]; q += kTailThreads) pr[q] = a.rows.pieces[q];
+  for (int q = threadIdx.x; q < a.cols.p0[kClasses]; q += kTailThreads) pc[q] = a.cols.pieces[q];
   unsigned target = 0;
   auto barrier = [&]() {
     return persist_barrier(a.counter, target += gridDim.x, a.err, a.budget, [] {});
@@ -566,40 +655,22 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_batch_tail(const __grid_con
   };
   if (!look()) return;
   for (int it = 0; it < n; ++it) {
-    int x = 0;
-    for (int i = gc; !__all_sync(0xffffffffu, i >= C); i += nc) {
-      while (i < C && i >= a.pcol[x + 1]) ++x;
-      const bool on = i < C && live[x];
-      const int64_t j = on ? a.col0[x] + (i - a.pcol[x]) : a.cols.nseg;
-      const double g = persist_group_sum(persist_dot_again<2>(a.cols, (int)j, lc, a.f.mr32), a.cols.L);
-      if (on && lc == 0) {
-        double v = a.u.x64[j] + a.u.lam[a.inst[x]] * (a.u.D[j] * g);
-        if (a.u.lbk) v = fmax(v, a.u.lb);
-        if (a.u.ubk) v = fmin(v, a.u.ub);
-        a.u.x64[j] = v;
-        a.u.x32[j] = (float)v;
-      }
-    }
+    tail_pass(a.cols, pc, live, a.row0, a.f.mr32, [&](int j, int x, double g) {
+      batch_update(j, g, a.u.x64[j], a.u.lam[a.inst[x]], a.u.D[j], a.u);
+    });
     if (!barrier()) return;
-    x = 0;
-    for (int i = gr; !__all_sync(0xffffffffu, i >= R); i += nr) {
-      while (i < R && i >= a.prow[x + 1]) ++x;
-      const bool on = i < R && live[x];
-      const int64_t r = on ? a.row0[x] + (i - a.prow[x]) : a.rows.nseg;
-      const double s = persist_group_sum(persist_dot_again<2>(a.rows, (int)r, lr, a.u.x32), a.rows.L);
-      if (on && lr == 0) {
-        const double ri = a.f.b[r] - s;
-        a.f.mr32[r] = (float)(a.f.M[r] * ri);
-        a.f.rsq[r] = ri * ri;
-      }
-    }
+    tail_pass(a.rows, pr, live, a.col0, a.u.x32,
+              [&](int r, int, double s) { batch_residual(r, s, a.f.b[r], a.f.M[r], a.f); });
     if (!barrier()) return;
     if (blockIdx.x < a.count && live[blockIdx.x]) {
       const int k = a.inst[blockIdx.x];
-      const int64_t r0 = a.row0[blockIdx.x], m = a.prow[blockIdx.x + 1] - a.prow[blockIdx.x];
+      const double *rsq = a.f.rsq + a.row0[blockIdx.x];
       double v = 0.0;
-      for (int64_t i = threadIdx.x; i < m; i += kTailThreads) v += a.f.rsq[r0 + i];
-      v = block_sum<kTailThreads>(v);
+      if (threadIdx.x < 256) {
+#pragma unroll 8
+        for (int i = threadIdx.x; i < a.m[blockIdx.x]; i += 256) v += rsq[i];
+      }
+      v = block_sum<kTailThreads>(v);  // the warps past 256 threads add zeros
       if (threadIdx.x == 0 && batch_rule(k, 0, a.kmax, a.c, v, a.iters, a.rule, a.resn)) a.stop[k] = 1;
     }
     if (!barrier()) return;
@@ -811,7 +882,8 @@ void setup_tileset(TileSet &T, int64_t nseg, const int64_t *ptr, cudaStream_t s)
   if (T.ntiles == 0) return;
   k_tile_class<<<(T.ntiles + 127) / 128, 128, 0, s>>>(T.ntiles, nseg, ptr, T.cls.p);
   AIRT_LAUNCH_CHECK();
-  std::vector<int> h(T.ntiles);
+  std::vector<int> &h = T.hcls;
+  h.resize(T.ntiles);
   AIRT_CHECK_CUDA(cudaMemcpyAsync(h.data(), T.cls.p, T.ntiles * sizeof(int), cudaMemcpyDeviceToHost, s));
   AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
   for (int v : h) ++T.count[v];
@@ -1136,15 +1208,50 @@ void batch_ncp_setup(Batch &B) {
 }  // namespace
 
 namespace {
+// The pieces of one direction for the instances a.inst (segments off[k] ..
+// off[k+1]); false when there are more than the kernel holds.
+bool tail_pieces(const TileSet &T, const TailArgs &a, const std::vector<int64_t> &off, int threads,
+                 std::vector<TailPiece> &out, TailDir &d) {
+  std::vector<TailPiece> by[kClasses];
+  for (int q = 0; q < a.count; ++q) {
+    const int64_t s0 = off[a.inst[q]], s1 = off[a.inst[q] + 1];
+    for (int64_t s = s0; s < s1;) {
+      const int64_t e = std::min(s1, ((s >> kTileShift) + 1) << kTileShift);
+      auto &v = by[T.hcls[s >> kTileShift]];
+      if (!v.empty() && v.back().slot == q && v.back().first + v.back().count == s) v.back().count += (int)(e - s);
+      else v.push_back(TailPiece{(int)s, (int)(e - s), 0, q});
+      s = e;
+    }
+  }
+  int64_t used = 0;  // threads taken by the classes before: another share of the grid for each
+  for (int c = 0; c < kClasses; ++c) {
+    d.p0[c] = (int)out.size();
+    int64_t n = 0;
+    for (TailPiece &p : by[c]) {
+      p.start = (int)n;
+      n += p.count;
+      out.push_back(p);
+    }
+    if (n >= (1 << 30)) return false;  // the kernel's counters run past the end by a grid
+    d.total[c] = (int)n;
+    d.lanes[c] = T.lanes[c];
+    d.shift[c] = (int)((used + 31) / 32 * 32 % threads);
+    used = d.shift[c] + n * d.lanes[c];
+  }
+  d.p0[kClasses] = (int)out.size();
+  return out.size() <= (size_t)kTailPieces;
+}
+
 // Runs the instances that have not stopped to the end in one launch, when they
 // are few and small enough: the flags are read back (the stream is drained).
 // done: iterations every running instance has behind it.  Returns whether it
-// did.
-bool batch_tail(Batch &B, const BFwd &fo, const BUpd &uo, const BCtrl &co, int64_t done, int64_t kmax) {
+// did; if not, *again is the number of running instances from which on their
+// nonzeros may be few enough.
+bool batch_tail(Batch &B, const BFwd &fo, const BUpd &uo, const BCtrl &co, int64_t done, int64_t kmax, int *again) {
   Problem &P = B.P;
   cudaStream_t s = P.stream;
   const int K = B.ninst;
-  if (P.m >= INT32_MAX || P.n >= INT32_MAX) return false;
+  *again = 0;
   if (B.inst_nnz.empty()) {
     DevBuf<int64_t> d;
     d.ensure(K + 1);
@@ -1159,32 +1266,46 @@ bool batch_tail(Batch &B, const BFwd &fo, const BUpd &uo, const BCtrl &co, int64
   std::vector<int> hstop(K);
   AIRT_CHECK_CUDA(cudaMemcpyAsync(hstop.data(), B.stop.p, K * sizeof(int), cudaMemcpyDeviceToHost, s));
   AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+  std::vector<int64_t> sizes;  // nonzeros of the running instances
+  for (int k = 0; k < K; ++k)
+    if (!hstop[k]) sizes.push_back(B.inst_nnz[k]);
+  if (sizes.empty()) return true;
+  std::sort(sizes.begin(), sizes.end());
+  int fit = 0;  // so many of the smallest are few enough together
+  for (int64_t sum = 0; fit < (int)sizes.size() && sum + sizes[fit] <= kTailNnz; ++fit) sum += sizes[fit];
+  *again = std::min(fit, kTailInst);
+  if (*again < (int)sizes.size()) return false;
+  *again = 0;
   TailArgs a{};
-  int64_t nnz = 0;
   for (int k = 0; k < K; ++k) {
     if (hstop[k]) continue;
-    if (a.count == kTailInst) return false;
-    const int64_t m = B.row_off[k + 1] - B.row_off[k], n = B.col_off[k + 1] - B.col_off[k];
     const int q = a.count++;
-    nnz += B.inst_nnz[k];
-    if (nnz > kTailNnz || a.prow[q] + m >= INT32_MAX || a.pcol[q] + n >= INT32_MAX) return false;
     a.inst[q] = k;
     a.row0[q] = B.row_off[k];
     a.col0[q] = B.col_off[k];
-    a.prow[q + 1] = a.prow[q] + (int)m;
-    a.pcol[q + 1] = a.pcol[q] + (int)n;
+    a.m[q] = (int)(B.row_off[k + 1] - B.row_off[k]);
   }
-  if (a.count == 0) return true;
   const unsigned grid = (unsigned)num_sms();
   if (a.count > (int)grid) return false;
   int occ = 0;
   AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_tail, kTailThreads, 0));
   if (occ < 1) return false;
-  auto lanes = [&](int64_t nseg) {
-    return persist_lanes(nnz, nseg, (int64_t)grid * kTailThreads);
-  };
-  a.rows = PersistDir{(int)P.m, P.rp.p, P.ci.p, P.rv.p, lanes(a.prow[a.count])};
-  a.cols = PersistDir{(int)P.n, P.cp.p, P.ri.p, P.cv.p, lanes(a.pcol[a.count])};
+  std::vector<TailPiece> pr, pc;
+  if (!tail_pieces(B.rt, a, B.row_off, (int)grid * kTailThreads, pr, a.rows) ||
+      !tail_pieces(B.ct, a, B.col_off, (int)grid * kTailThreads, pc, a.cols))
+    return false;
+  B.tail_pr.upload(pr.data(), pr.size(), s);
+  B.tail_pc.upload(pc.data(), pc.size(), s);
+  a.rows.ptr = P.rp.p;
+  a.rows.idx = P.ci.p;
+  a.rows.idx16 = B.ci16.p;
+  a.rows.val = P.rv.p;
+  a.rows.pieces = B.tail_pr.p;
+  a.cols.ptr = P.cp.p;
+  a.cols.idx = P.ri.p;
+  a.cols.idx16 = B.ri16.p;
+  a.cols.val = P.cv.p;
+  a.cols.pieces = B.tail_pc.p;
   a.f = fo;
   a.u = uo;
   a.c = co;
@@ -1318,16 +1439,12 @@ void batch_sirt(Batch &B, int method, const double *lam_host, const double *d_b,
   const int64_t chunk = 8;
   const int lag = 2;
   // rules whose last instances may finish in one launch, and the active count
-  // at which that was last tried in vain.  A solve of a few iterations is done
-  // before the flags would be back, and its first iterate stays the
-  // back projection bit for bit.
+  // from which on that is worth a try (it drains the stream).  A solve of a
+  // few iterations is done before the flags would be back.
   const bool tail_ok = !me && !ncp && kmax >= chunk;
-  int tried = K + 1;
+  int again = kTailInst;
   bool finished = false;
-  if (tail_ok && K <= kTailInst) {
-    finished = batch_tail(B, fo, uo, co, 0, kmax);
-    tried = K;
-  }
+  if (tail_ok && K <= again) finished = batch_tail(B, fo, uo, co, 0, kmax, &again);
   cudaGraphExec_t gexec = nullptr;
   if (kmax >= chunk && !finished) {
     cudaGraph_t g = nullptr;
@@ -1361,10 +1478,7 @@ void batch_sirt(Batch &B, int method, const double *lam_host, const double *d_b,
       AIRT_CHECK_CUDA(cudaEventSynchronize(ev[(c - lag) % 3]));
       const int act = hact[(c - lag) % 3];
       if (act == 0) break;
-      if (tail_ok && act <= kTailInst && act < tried && it <= kmax) {
-        finished = batch_tail(B, fo, uo, co, it - 1, kmax);
-        tried = act;
-      }
+      if (tail_ok && act <= again && it <= kmax) finished = batch_tail(B, fo, uo, co, it - 1, kmax, &again);
     }
   }
   for (int q = 0; q < 3; ++q) cudaEventDestroy(ev[q]);

@@ -182,6 +182,93 @@ __device__ __forceinline__ void for_each_segment_vpre(int64_t nseg, const int64_
   }
 }
 
+// One element of the gathered vector.  LIVE: the vector changes while the
+// kernel runs (between grid barriers), so it is not read through the
+// read-only path.
+template <bool LIVE, typename TX>
+__device__ __forceinline__ TX gathered(const TX *p) {
+  return LIVE ? *p : __ldg(p);
+}
+
+// A lane's part of the sum over nonzeros [q0, q1): every aligned 16-byte
+// group that overlaps them, its elements outside masked out (they belong to
+// the neighbouring segments or the zero padding, so the loads stay inside the
+// arrays): no element-wise head or tail loop, which on short segments (tens
+// of nonzeros) would hold a large share of the loads in serial chains.
+template <int LANES, bool LIVE, typename TX>
+__device__ __forceinline__ double segment_part(int64_t q0, int64_t q1, int lane, const int *idx, const float *val,
+                                               const TX *x) {
+  const float4 *V4 = reinterpret_cast<const float4 *>(val);
+  const int4 *I4 = reinterpret_cast<const int4 *>(idx);
+  auto get = [&](int c) { return gathered<LIVE>(x + c); };
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+  const int64_t ve = (q1 + 3) >> 2;
+  int64_t v = (q0 >> 2) + lane;
+  for (; v + LANES < ve; v += 2 * LANES) {
+    const float4 f = __ldg(V4 + v), h = __ldg(V4 + v + LANES);
+    const int4 c = __ldg(I4 + v), d = __ldg(I4 + v + LANES);
+    const TX g0 = get(c.x), g1 = get(c.y), g2 = get(c.z), g3 = get(c.w);
+    const TX k0 = get(d.x), k1 = get(d.y), k2 = get(d.z), k3 = get(d.w);
+    const int64_t e = v << 2, e2 = (v + LANES) << 2;
+    if (e >= q0 && e < q1) a0 = fma((double)f.x, (double)g0, a0);
+    if (e + 1 >= q0 && e + 1 < q1) a1 = fma((double)f.y, (double)g1, a1);
+    if (e + 2 >= q0 && e + 2 < q1) a2 = fma((double)f.z, (double)g2, a2);
+    if (e + 3 >= q0 && e + 3 < q1) a3 = fma((double)f.w, (double)g3, a3);
+    if (e2 < q1) a0 = fma((double)h.x, (double)k0, a0);
+    if (e2 + 1 < q1) a1 = fma((double)h.y, (double)k1, a1);
+    if (e2 + 2 < q1) a2 = fma((double)h.z, (double)k2, a2);
+    if (e2 + 3 < q1) a3 = fma((double)h.w, (double)k3, a3);
+  }
+  if (v < ve) {
+    const float4 f = __ldg(V4 + v);
+    const int4 c = __ldg(I4 + v);
+    const TX g0 = get(c.x), g1 = get(c.y), g2 = get(c.z), g3 = get(c.w);
+    const int64_t e = v << 2;
+    if (e >= q0 && e < q1) a0 = fma((double)f.x, (double)g0, a0);
+    if (e + 1 >= q0 && e + 1 < q1) a1 = fma((double)f.y, (double)g1, a1);
+    if (e + 2 >= q0 && e + 2 < q1) a2 = fma((double)f.z, (double)g2, a2);
+    if (e + 3 >= q0 && e + 3 < q1) a3 = fma((double)f.w, (double)g3, a3);
+  }
+  return (a0 + a1) + (a2 + a3);
+}
+
+// The same with 16-bit indices: 8 nonzeros per 16-byte index load (two float4
+// value loads), so the streamed bytes per nonzero drop from 8 to 6.  The
+// 8-aligned body is vectorised, the head and tail (< 8 elements each) are read
+// element-wise.
+template <int LANES, bool LIVE, typename TX>
+__device__ __forceinline__ double segment_part16(int64_t q0, int64_t q1, int lane, const uint16_t *idx,
+                                                 const float *val, const TX *x) {
+  const float4 *V4 = reinterpret_cast<const float4 *>(val);
+  const uint4 *I8 = reinterpret_cast<const uint4 *>(idx);
+  auto get = [&](unsigned c) { return gathered<LIVE>(x + c); };
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+  int64_t qa = (q0 + 7) & ~(int64_t)7;
+  if (qa > q1) qa = q1;
+  int64_t qb = q1 & ~(int64_t)7;
+  if (qb < qa) qb = qa;
+  for (int64_t q = q0 + lane; q < qa; q += LANES) a0 = fma((double)__ldg(val + q), (double)get(__ldg(idx + q)), a0);
+  for (int64_t q = qb + lane; q < q1; q += LANES) a1 = fma((double)__ldg(val + q), (double)get(__ldg(idx + q)), a1);
+  const int64_t ge = qb >> 3;
+  for (int64_t gq = (qa >> 3) + lane; gq < ge; gq += LANES) {
+    const uint4 c = __ldg(I8 + gq);
+    const float4 f = __ldg(V4 + 2 * gq), h = __ldg(V4 + 2 * gq + 1);
+    const TX g0 = get(c.x & 0xFFFFu), g1 = get(c.x >> 16);
+    const TX g2 = get(c.y & 0xFFFFu), g3 = get(c.y >> 16);
+    const TX g4 = get(c.z & 0xFFFFu), g5 = get(c.z >> 16);
+    const TX g6 = get(c.w & 0xFFFFu), g7 = get(c.w >> 16);
+    a0 = fma((double)f.x, (double)g0, a0);
+    a1 = fma((double)f.y, (double)g1, a1);
+    a2 = fma((double)f.z, (double)g2, a2);
+    a3 = fma((double)f.w, (double)g3, a3);
+    a0 = fma((double)h.x, (double)g4, a0);
+    a1 = fma((double)h.y, (double)g5, a1);
+    a2 = fma((double)h.z, (double)g6, a2);
+    a3 = fma((double)h.w, (double)g7, a3);
+  }
+  return (a0 + a1) + (a2 + a3);
+}
+
 // for_each_segment_v over a list of segment tiles, with a per-segment
 // predicate.  Tile t covers segments t << tshift .. +(1 << tshift); the
 // groups walk the *ntiles listed tiles (tiles[0 .. *ntiles)), so ranges left
@@ -206,8 +293,6 @@ __device__ __forceinline__ void for_each_segment_vt(int64_t nseg, const int *__r
   const int64_t total = (int64_t)__ldg(ntiles) << tshift;
   const int64_t tmask = ((int64_t)1 << tshift) - 1;
   const int64_t trips = (total + ng - 1) / ng;
-  const float4 *__restrict__ V4 = reinterpret_cast<const float4 *>(val);
-  const int4 *__restrict__ I4 = reinterpret_cast<const int4 *>(idx);
   for (int64_t t = 0; t < trips; ++t) {
     const int64_t u = gid + t * ng;
     const int64_t i = u < total ? ((int64_t)__ldg(tiles + (u >> tshift)) << tshift) + (u & tmask) : nseg;
@@ -220,42 +305,7 @@ __device__ __forceinline__ void for_each_segment_vt(int64_t nseg, const int *__r
       on = active(i);
       if (on && lane == 0) pv = pre(i);
     }
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    if (on) {
-      // every aligned 16-byte group that overlaps [q0, q1), its elements
-      // outside the segment masked out (they belong to the neighbouring
-      // segments or the zero padding, so the loads stay inside the arrays):
-      // no element-wise head or tail loop, which on short segments (tens of
-      // nonzeros) would hold a large share of the loads in serial chains
-      const int64_t ve = (q1 + 3) >> 2;
-      int64_t v = (q0 >> 2) + lane;
-      for (; v + LANES < ve; v += 2 * LANES) {
-        const float4 f = __ldg(V4 + v), h = __ldg(V4 + v + LANES);
-        const int4 c = __ldg(I4 + v), d = __ldg(I4 + v + LANES);
-        const TX g0 = __ldg(x + c.x), g1 = __ldg(x + c.y), g2 = __ldg(x + c.z), g3 = __ldg(x + c.w);
-        const TX k0 = __ldg(x + d.x), k1 = __ldg(x + d.y), k2 = __ldg(x + d.z), k3 = __ldg(x + d.w);
-        const int64_t e = v << 2, e2 = (v + LANES) << 2;
-        if (e >= q0 && e < q1) a0 = fma((double)f.x, (double)g0, a0);
-        if (e + 1 >= q0 && e + 1 < q1) a1 = fma((double)f.y, (double)g1, a1);
-        if (e + 2 >= q0 && e + 2 < q1) a2 = fma((double)f.z, (double)g2, a2);
-        if (e + 3 >= q0 && e + 3 < q1) a3 = fma((double)f.w, (double)g3, a3);
-        if (e2 < q1) a0 = fma((double)h.x, (double)k0, a0);
-        if (e2 + 1 < q1) a1 = fma((double)h.y, (double)k1, a1);
-        if (e2 + 2 < q1) a2 = fma((double)h.z, (double)k2, a2);
-        if (e2 + 3 < q1) a3 = fma((double)h.w, (double)k3, a3);
-      }
-      if (v < ve) {
-        const float4 f = __ldg(V4 + v);
-        const int4 c = __ldg(I4 + v);
-        const TX g0 = __ldg(x + c.x), g1 = __ldg(x + c.y), g2 = __ldg(x + c.z), g3 = __ldg(x + c.w);
-        const int64_t e = v << 2;
-        if (e >= q0 && e < q1) a0 = fma((double)f.x, (double)g0, a0);
-        if (e + 1 >= q0 && e + 1 < q1) a1 = fma((double)f.y, (double)g1, a1);
-        if (e + 2 >= q0 && e + 2 < q1) a2 = fma((double)f.z, (double)g2, a2);
-        if (e + 3 >= q0 && e + 3 < q1) a3 = fma((double)f.w, (double)g3, a3);
-      }
-    }
-    double acc = (a0 + a1) + (a2 + a3);
+    double acc = on ? segment_part<LANES, false>(q0, q1, lane, idx, val, x) : 0.0;
     acc = group_sum<LANES>(acc);
     epi(i, acc, lane == 0 && on, pv);
   }
@@ -264,11 +314,7 @@ __device__ __forceinline__ void for_each_segment_vt(int64_t nseg, const int *__r
 // for_each_segment_vt over a block-diagonal matrix whose indices are stored
 // as 16-bit offsets within each segment's instance: segment i belongs to
 // instance inst_of[i], runs when stop[that] == 0, and gathers x[voff[that] +
-// local index].  A lane reads 8 nonzeros per 16-byte index load (two float4
-// value loads), two such groups per round, so the streamed bytes per
-// nonzero drop from 8 to 6.  The 8-aligned body is vectorised, the head and
-// tail (< 8 elements each) are read element-wise; segment sums run in a
-// fixed order (per lane four accumulators, then the group's shuffle tree).
+// local index] (segment_part16).
 template <int LANES, typename TX, class Pre, class Epi>
 __device__ __forceinline__ void for_each_segment_vt16(int64_t nseg, const int *__restrict__ tiles,
                                                       const int *__restrict__ ntiles, int tshift,
@@ -286,8 +332,6 @@ __device__ __forceinline__ void for_each_segment_vt16(int64_t nseg, const int *_
   const int64_t total = (int64_t)__ldg(ntiles) << tshift;
   const int64_t tmask = ((int64_t)1 << tshift) - 1;
   const int64_t trips = (total + ng - 1) / ng;
-  const float4 *__restrict__ V4 = reinterpret_cast<const float4 *>(val);
-  const uint4 *__restrict__ I8 = reinterpret_cast<const uint4 *>(idx);
   for (int64_t t = 0; t < trips; ++t) {
     const int64_t u = gid + t * ng;
     const int64_t i = u < total ? ((int64_t)__ldg(tiles + (u >> tshift)) << tshift) + (u & tmask) : nseg;
@@ -303,36 +347,7 @@ __device__ __forceinline__ void for_each_segment_vt16(int64_t nseg, const int *_
       xb = x + __ldg(voff + k);
       if (on && lane == 0) pv = pre(i);
     }
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    if (on) {
-      int64_t qa = (q0 + 7) & ~(int64_t)7;
-      if (qa > q1) qa = q1;
-      int64_t qb = q1 & ~(int64_t)7;
-      if (qb < qa) qb = qa;
-      for (int64_t q = q0 + lane; q < qa; q += LANES)
-        a0 = fma((double)__ldg(val + q), (double)__ldg(xb + __ldg(idx + q)), a0);
-      for (int64_t q = qb + lane; q < q1; q += LANES)
-        a1 = fma((double)__ldg(val + q), (double)__ldg(xb + __ldg(idx + q)), a1);
-      const int64_t ge = qb >> 3;
-      int64_t gq = (qa >> 3) + lane;
-      for (; gq < ge; gq += LANES) {
-        const uint4 c = __ldg(I8 + gq);
-        const float4 f = __ldg(V4 + 2 * gq), h = __ldg(V4 + 2 * gq + 1);
-        const TX g0 = __ldg(xb + (c.x & 0xFFFFu)), g1 = __ldg(xb + (c.x >> 16));
-        const TX g2 = __ldg(xb + (c.y & 0xFFFFu)), g3 = __ldg(xb + (c.y >> 16));
-        const TX g4 = __ldg(xb + (c.z & 0xFFFFu)), g5 = __ldg(xb + (c.z >> 16));
-        const TX g6 = __ldg(xb + (c.w & 0xFFFFu)), g7 = __ldg(xb + (c.w >> 16));
-        a0 = fma((double)f.x, (double)g0, a0);
-        a1 = fma((double)f.y, (double)g1, a1);
-        a2 = fma((double)f.z, (double)g2, a2);
-        a3 = fma((double)f.w, (double)g3, a3);
-        a0 = fma((double)h.x, (double)g4, a0);
-        a1 = fma((double)h.y, (double)g5, a1);
-        a2 = fma((double)h.z, (double)g6, a2);
-        a3 = fma((double)h.w, (double)g7, a3);
-      }
-    }
-    double acc = (a0 + a1) + (a2 + a3);
+    double acc = on ? segment_part16<LANES, false>(q0, q1, lane, idx, val, xb) : 0.0;
     acc = group_sum<LANES>(acc);
     epi(i, acc, lane == 0 && on, pv);
   }
