@@ -5,7 +5,7 @@ method wrappers, the ``paralleltomo``/``fanlineartomo`` test problems and the
 afun operator handle.  All iterations run in libairt.so (hand-written CUDA for
 sm_100a); the package raises on import if the library is missing.
 """
-from ._lib import AirtError, lib as _load_lib
+from ._lib import AirtError, lib as _load_lib, release_memory
 from .afun import AirtOperator, afun_matrix, as_operator
 from .batch import ParallelBatch
 from .analytic import fbp
@@ -21,4 +21,4 @@ __all__ = ["AirtError", "AirtOperator", "ParallelBatch", "UNet", "afun_matrix", 
            "cimmino", "drop", "kaczmarz", "landweber", "randkaczmarz", "sart", "sirt",
            "symkaczmarz", "add_noise", "cosd", "fancurvedtomo", "fanlineartomo", "paralleltomo", "seismictomo",
            "sphericaltomo",
-           "phantomgallery", "random_ellipses", "sind"]
+           "phantomgallery", "random_ellipses", "release_memory", "sind"]

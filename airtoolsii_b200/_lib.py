@@ -147,6 +147,10 @@ SIGNATURES = {
     "airt_residual_noalloc": (C.c_int, [C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
                                         C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                         C.c_void_p]),
+    "airt_release_memory": (C.c_int, []),
+    "airt_test_pool_new": (C.c_void_p, [C.c_int64]),
+    "airt_test_pool_op": (C.c_int64, [C.c_void_p, C.c_int, C.c_int64]),
+    "airt_test_pool_delete": (None, [C.c_void_p]),
     "airt_profile_enable": (C.c_int, [C.c_void_p, C.c_int]),
     "airt_profile_read": (C.c_int, [C.c_void_p, C.c_int, _i64p, _dp]),
 }
@@ -184,6 +188,12 @@ def check(status: int) -> None:
     if status != AIRT_OK:
         msg = lib().airt_last_error()
         raise AirtError(status, msg.decode() if msg else "")
+
+
+def release_memory() -> None:
+    """Give the device memory kept from destroyed handles back (all that is
+    kept in the current CUDA context), for another library's use."""
+    check(lib().airt_release_memory())
 
 
 def dptr(a):

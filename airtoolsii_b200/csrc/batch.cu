@@ -1006,7 +1006,7 @@ void batch_destroy(Batch *B) {
   if (!B) return;
   cudaStream_t s = B->P.stream;
   if (s) cudaStreamSynchronize(s);
-  pinned_free(B->P.h_state);
+  if (B->P.h_state) pinned_free(B->P.h_block);
   B->P.h_state = nullptr;
   delete B;
   if (s) cudaStreamDestroy(s);

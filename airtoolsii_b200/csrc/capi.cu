@@ -86,7 +86,7 @@ static void free_problem(Problem *P) {
     cudaEventDestroy(it.second.second);
   }
   for (auto e : P->ev_pool) cudaEventDestroy(e);
-  pinned_free(P->h_state);
+  if (P->h_state) pinned_free(P->h_block);
   cudaStream_t s = P->stream;
   delete P;
   if (s) cudaStreamDestroy(s);

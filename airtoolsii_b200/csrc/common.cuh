@@ -48,41 +48,52 @@ void set_error(const char *fmt, ...);
 // device were out of memory.
 extern int g_alloc_fail_countdown;
 
+// Id of the current CUDA context (noalloc.cu); throws when there is none.
+unsigned long long current_context_id();
+
 // Device memory for DevBuf (pool.cu): blocks that are given up are kept for
-// the next allocation of about their size.  device_alloc returns null when
-// the device is out of memory (*err then holds CUDA's error).  device_free
-// waits for the device, as cudaFree does, so a kept block is idle.
-void *device_alloc(size_t bytes, cudaError_t *err);
-void device_free(void *p);
+// the next allocation of about their size in the same context.  device_alloc
+// returns a null block when the device is out of memory (*err then holds
+// CUDA's error).  device_free waits for the device, as cudaFree does, so a
+// kept block is idle.
+struct DevBlock {
+  void *p = nullptr;
+  size_t size = 0;
+  unsigned long long ctx = 0;
+};
+DevBlock device_alloc(size_t bytes, cudaError_t *err);
+void device_free(const DevBlock &b) noexcept;
 // One page-locked buffer of kPinnedBytes, kept likewise.
 constexpr size_t kPinnedBytes = 1024;
-void *pinned_alloc(cudaError_t *err);
-void pinned_free(void *p);
+DevBlock pinned_alloc(cudaError_t *err);
+void pinned_free(const DevBlock &b) noexcept;
 
 template <typename T>
 struct DevBuf {
   T *p = nullptr;
   size_t n = 0;
+  DevBlock block;  // p's memory
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
-  DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n) {
-    o.p = nullptr;
-    o.n = 0;
-  }
+  DevBuf(DevBuf &&o) noexcept { take(o); }
   DevBuf &operator=(DevBuf &&o) noexcept {
     if (this != &o) {
       release();
-      p = o.p;
-      n = o.n;
-      o.p = nullptr;
-      o.n = 0;
+      take(o);
     }
     return *this;
   }
   ~DevBuf() { release(); }
+  void take(DevBuf &o) noexcept {
+    p = o.p;
+    n = o.n;
+    block = o.block;
+    o.p = nullptr;
+    o.n = 0;
+  }
   void release() {
-    if (p) device_free(p);
+    if (p) device_free(block);
     p = nullptr;
     n = 0;
   }
@@ -96,7 +107,8 @@ struct DevBuf {
       throw Status{AIRT_ERR_OOM};
     }
     cudaError_t e = cudaSuccess;
-    p = static_cast<T *>(device_alloc(bytes, &e));
+    block = device_alloc(bytes, &e);
+    p = static_cast<T *>(block.p);
     if (!p) {
       set_error("cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
       throw Status{AIRT_ERR_OOM};
@@ -282,6 +294,7 @@ struct Problem {
   DevBuf<unsigned> pst_count;
   DevBuf<int> save_slot;
   SirtState *h_state = nullptr;  // pinned mirror (3 entries)
+  DevBlock h_block;              // its memory
 
   // instrumentation
   bool profiling = false;
@@ -322,8 +335,10 @@ inline void ensure_h_state(Problem &P) {
   static_assert(3 * sizeof(SirtState) <= kPinnedBytes, "pinned mirror");
   if (P.h_state) return;
   cudaError_t e = cudaSuccess;
-  P.h_state = static_cast<SirtState *>(pinned_alloc(&e));
+  const DevBlock b = pinned_alloc(&e);
   AIRT_CHECK_CUDA(e);
+  P.h_block = b;
+  P.h_state = static_cast<SirtState *>(b.p);
 }
 
 inline int num_sms() {

@@ -117,38 +117,40 @@ __global__ void k_noalloc_finish(const double *__restrict__ acc, const int *__re
                                                       : sqrt(*acc);
 }
 
-using PFN_ctxGetCurrent = CUresult(CUDAAPI *)(CUcontext *);
-using PFN_ctxGetId = CUresult(CUDAAPI *)(CUcontext, unsigned long long *);
+}  // namespace
 
 // The current context's id, through the driver entry points the runtime
 // hands out (the library does not link libcuda).  Makes the device's primary
 // context current first when the calling thread has no context, as any
 // runtime call would.
 unsigned long long current_context_id() {
-  static PFN_ctxGetCurrent get_current = nullptr;
-  static PFN_ctxGetId get_id = nullptr;
-  if (!get_current || !get_id) {
+  struct Entry {
+    CUresult(CUDAAPI *get_current)(CUcontext *);
+    CUresult(CUDAAPI *get_id)(CUcontext, unsigned long long *);
+  };
+  static const Entry e = [] {
     void *f1 = nullptr, *f2 = nullptr;
     cudaDriverEntryPointQueryResult q1, q2;
     AIRT_CHECK_CUDA(cudaGetDriverEntryPoint("cuCtxGetCurrent", &f1, cudaEnableDefault, &q1));
     AIRT_CHECK_CUDA(cudaGetDriverEntryPoint("cuCtxGetId", &f2, cudaEnableDefault, &q2));
     AIRT_REQUIRE(q1 == cudaDriverEntryPointSuccess && q2 == cudaDriverEntryPointSuccess && f1 && f2,
                  "the CUDA driver does not provide cuCtxGetCurrent/cuCtxGetId");
-    get_current = reinterpret_cast<PFN_ctxGetCurrent>(f1);
-    get_id = reinterpret_cast<PFN_ctxGetId>(f2);
-  }
+    return Entry{reinterpret_cast<decltype(Entry::get_current)>(f1), reinterpret_cast<decltype(Entry::get_id)>(f2)};
+  }();
   CUcontext ctx = nullptr;
-  if (get_current(&ctx) != CUDA_SUCCESS || !ctx) {
+  if (e.get_current(&ctx) != CUDA_SUCCESS || !ctx) {
     int dev = 0;
     AIRT_CHECK_CUDA(cudaGetDevice(&dev));
     AIRT_CHECK_CUDA(cudaSetDevice(dev));   // binds the device's primary context
     ctx = nullptr;
-    AIRT_REQUIRE(get_current(&ctx) == CUDA_SUCCESS && ctx, "no current CUDA context");
+    AIRT_REQUIRE(e.get_current(&ctx) == CUDA_SUCCESS && ctx, "no current CUDA context");
   }
   unsigned long long id = 0;
-  AIRT_REQUIRE(get_id(ctx, &id) == CUDA_SUCCESS, "cuCtxGetId failed");
+  AIRT_REQUIRE(e.get_id(ctx, &id) == CUDA_SUCCESS, "cuCtxGetId failed");
   return id;
 }
+
+namespace {
 
 unsigned char *scratch_address() {
   const unsigned long long id = current_context_id();

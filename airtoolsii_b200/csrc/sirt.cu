@@ -1304,8 +1304,7 @@ double estimate_rho(Problem &P, const double *dM, const double *dD, double tol, 
     prev = theta;
     beta.push_back(b);
     inv_b = 1.0 / b;
-    std::swap(vprev.p, v.p);
-    std::swap(vprev.n, v.n);
+    std::swap(vprev, v);
   }
   return theta;
 }

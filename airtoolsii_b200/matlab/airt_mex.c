@@ -497,6 +497,14 @@ static void cmd_destroy(int nlhs, mxArray *plhs[], int nrhs, const mxArray *prhs
     (void)plhs;
 }
 
+static void cmd_release_memory(int nlhs, mxArray *plhs[], int nrhs, const mxArray *prhs[]) {
+    need(nrhs == 1, "airt_mex('release_memory')");
+    chk(airt_release_memory());
+    (void)nlhs;
+    (void)plhs;
+    (void)prhs;
+}
+
 /* ---- batches: a batch travels as its handle plus its instance count */
 static const int *ivec(const mxArray *a, int64_t *count) {
     need(a && mxIsInt32(a), "expected an int32 array");
@@ -788,6 +796,7 @@ static const struct command commands[] = {
     {"cart", cmd_cart},
     {"fbp", cmd_fbp},
     {"destroy", cmd_destroy},
+    {"release_memory", cmd_release_memory},
     {"batch", cmd_batch},
     {"batch_layout", cmd_batch_layout},
     {"batch_rho", cmd_batch_rho},

@@ -379,6 +379,13 @@ int airt_residual_noalloc(int64_t m, int64_t n, const int64_t *d_rp, const int *
                           const float *d_rv, const double *d_x, const double *d_b, double *d_r,
                           double *d_resnorm, void *cuda_stream);
 
+/* ---- device memory --------------------------------------------------------- */
+/* No counterpart in the reference.  Memory of destroyed handles is kept for
+ * the next ones: per CUDA context, at most 6 GB and a quarter of the free
+ * memory, at most about 30 s between calls.  This gives all that is kept in
+ * the current context back to the device, for another library's use. */
+int airt_release_memory(void);
+
 /* ---- test hooks ----------------------------------------------------------- */
 /* No counterpart in the reference.  For tests of the bounded device waits:
  * airt_test_set_wait_budget sets the clock64 cycle budget of each wait of the
@@ -397,6 +404,16 @@ int airt_test_fail_alloc(int after);
  * matrix-free kernels trace on two threads (count and an order-independent
  * hash); *mismatched = rays that differ, *split = rays that were split. */
 int airt_test_split_trace(airt_problem *h, int64_t *mismatched, int64_t *split);
+
+/* The bookkeeping of the kept memory over a made-up device of `bytes` bytes.
+ * op: 0 context id = arg, 1 waiting for the device succeeds (arg != 0),
+ * 2 arg seconds pass, 3 context arg and its memory are gone, 4 allocate arg
+ * bytes (block number or -1), 5 give block arg up, 6 release, 7 address of
+ * block arg, 8 device allocations, 9 device frees, 10 frees of an address that
+ * is not allocated, 11 bytes taken from the device. */
+void *airt_test_pool_new(int64_t bytes);
+int64_t airt_test_pool_op(void *pool, int op, int64_t arg);
+void airt_test_pool_delete(void *pool);
 
 /* ---- instrumentation ------------------------------------------------------- */
 /* When on, each SIRT kernel launch is bracketed by CUDA events on the problem
