@@ -1446,17 +1446,10 @@ void batch_sirt(Batch &B, int method, const double *lam_host, const double *d_b,
   bool finished = false;
   if (tail_ok && K <= again) finished = batch_tail(B, fo, uo, co, 0, kmax, &again);
   cudaGraphExec_t gexec = nullptr;
-  if (kmax >= chunk && !finished) {
-    cudaGraph_t g = nullptr;
-    AIRT_CHECK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int64_t j = 0; j < chunk; ++j) iteration();
-    const cudaError_t ec = cudaStreamEndCapture(s, &g);
-    if (ec == cudaSuccess && g) {
-      if (cudaGraphInstantiate(&gexec, g, 0) != cudaSuccess) gexec = nullptr;
-      cudaGraphDestroy(g);
-    }
-    cudaGetLastError();
-  }
+  if (kmax >= chunk && !finished)
+    gexec = capture_graph(s, [&] {
+      for (int64_t j = 0; j < chunk; ++j) iteration();
+    });
   ensure_h_state(P);
   int *hact = reinterpret_cast<int *>(P.h_state);  // 3 poll slots in the pinned mirror
   cudaEvent_t ev[3];

@@ -331,6 +331,30 @@ struct Problem {
 };
 
 // ---------------------------------------------------------------- helpers
+// Captures what enqueue() launches on `s` as a graph.  Returns null when the
+// driver does not instantiate it; an exception in enqueue() ends the capture
+// before it goes on, so that the stream stays usable.
+template <class F>
+cudaGraphExec_t capture_graph(cudaStream_t s, F &&enqueue) {
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  AIRT_CHECK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  try {
+    enqueue();
+  } catch (...) {
+    cudaStreamEndCapture(s, &g);
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+    throw;
+  }
+  if (cudaStreamEndCapture(s, &g) == cudaSuccess && g) {
+    if (cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) exec = nullptr;
+    cudaGraphDestroy(g);
+  }
+  cudaGetLastError();
+  return exec;
+}
+
 inline void ensure_h_state(Problem &P) {
   static_assert(3 * sizeof(SirtState) <= kPinnedBytes, "pinned mirror");
   if (P.h_state) return;

@@ -514,19 +514,13 @@ void multi_pass(Problem &P, const airt_sirt_opts &o, int K0, const double *d_B, 
     if (gexec) cudaGraphExecDestroy(gexec);
     gexec = nullptr;
     if (kmax < chunk) return;
-    cudaGraph_t g = nullptr;
-    AIRT_CHECK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int64_t j = 0; j < chunk; ++j) {
-      bwd();
-      fwd();
-      ctrl(0);
-    }
-    const cudaError_t ec = cudaStreamEndCapture(s, &g);
-    if (ec == cudaSuccess && g) {
-      if (cudaGraphInstantiate(&gexec, g, 0) != cudaSuccess) gexec = nullptr;
-      cudaGraphDestroy(g);
-    }
-    cudaGetLastError();
+    gexec = capture_graph(s, [&] {
+      for (int64_t j = 0; j < chunk; ++j) {
+        bwd();
+        fwd();
+        ctrl(0);
+      }
+    });
   };
   capture();
   ensure_h_state(P);

@@ -711,7 +711,6 @@ void launch_fwd_t(Problem &P, const FwdOut &o) {
       return;
     }
     if (P.nslow) {
-      P.slow_y.ensure(P.m);
       k_sirt_slow_rows<<<(unsigned)((2 * (int64_t)P.nslow + 63) / 64), 64, 0, s>>>(
           P.geom(), P.nslow, excl, P.slow_rays.p, P.x32.p, P.slow_y.p, o.st);
     }
@@ -1056,18 +1055,12 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
   cudaGraphExec_t chunk_graph = nullptr;
   bool captured = P.profiling;
   auto capture = [&]() {
-    cudaGraph_t g = nullptr;
-    AIRT_CHECK_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int64_t j = 0; j < chunk; ++j) {
-      launch_bwd(P, ua, o.relax_kind, Dfull);
-      fwd();
-    }
-    const cudaError_t ec = cudaStreamEndCapture(s, &g);
-    if (ec == cudaSuccess && g) {
-      if (cudaGraphInstantiate(&chunk_graph, g, 0) != cudaSuccess) chunk_graph = nullptr;
-      cudaGraphDestroy(g);
-    }
-    cudaGetLastError();
+    chunk_graph = capture_graph(s, [&] {
+      for (int64_t j = 0; j < chunk; ++j) {
+        launch_bwd(P, ua, o.relax_kind, Dfull);
+        fwd();
+      }
+    });
     captured = true;
   };
   int64_t c = 0;

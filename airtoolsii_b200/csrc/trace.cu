@@ -443,7 +443,6 @@ void dda_adjoint(Problem &P, const TU *u, double *out, const unsigned long long 
   cudaStream_t s = P.stream;
   const unsigned g_ = (unsigned)((P.m + 31) / 32), t_ = 32u * dda_parts(P.m);
   unsigned long long *acc = reinterpret_cast<unsigned long long *>(out);
-  P.fxt.ensure(P.n);
   unsigned long long *acct = reinterpret_cast<unsigned long long *>(P.fxt.p);
   AIRT_CHECK_CUDA(cudaMemsetAsync(acc, 0, P.n * sizeof(double), s));
   AIRT_CHECK_CUDA(cudaMemsetAsync(acct, 0, P.n * sizeof(double), s));
@@ -601,6 +600,13 @@ void mf_prepare(Problem &P) {
   P.mf_kbound = T * (vmax > 0.0 ? vmax : 1.0);
   P.mf_umax.ensure(1);
   par_prepare(P);
+  // what the products and the iterations of a solve write beside their
+  // operands: none of them allocates, so that they can be captured
+  if (straight(P)) {
+    P.x64t.ensure(P.n);
+    if (!P.par_ok) P.fxt.ensure(P.n);
+    if (P.nslow) P.slow_y.ensure(P.m);
+  }
 }
 
 ParGather par_gather_of(const Problem &P) {
@@ -614,7 +620,6 @@ void apply_matrix_free(Problem &P, const double *d_in, double *d_out, int transp
   if (!transp) {
     if (P.m == 0) return;
     if (straight(P)) {
-      P.x64t.ensure(P.n);
       const unsigned tn = (unsigned)((P.N + 31) / 32);
       k_transpose_img<double><<<dim3(tn, tn), dim3(32, 8), 0, s>>>(P.N, d_in, P.x64t.p);
       AIRT_DDA_LAUNCH(k_dda_forward, d_in, P.x64t.p, d_out);
