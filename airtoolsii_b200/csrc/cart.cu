@@ -689,8 +689,9 @@ __global__ void __launch_bounds__(kCartBlockThreads) k_cart_block(CartArgs a, Ca
       // skipped columns and lanes past the end: a step clipped to [0, 0]
       const bool on = j >= 0 && non;
       const double c = on ? a.lam / nn : 0.0;
-      const double lo = on ? (lbon ? __dsub_rn(nlo, xj) : -INFINITY) : 0.0;
       const double hi = on ? (ubon ? __dsub_rn(nhi, xj) : INFINITY) : 0.0;
+      double lo = on ? (lbon ? __dsub_rn(nlo, xj) : -INFINITY) : 0.0;
+      if (lo > hi) lo = hi;  // the upper bound is applied last
       load_next(b + 1);
       const double *Gb = G + (b & 1) * kG + lane;
       double d = dots[b & 1][lane];
@@ -995,12 +996,13 @@ void run_cart(Problem &P, const airt_cart_opts &o, const double *d_b, const doub
     nrm.upload(hn.data(), n, s);
   }
   // the blocked sweep needs an order without repeats, (block, row) keys of
-  // 32 bits and rows of 27; its inner products take 512 bytes per column
+  // 32 bits, rows of 27 and a finite relaxpar/||a_j||^2; its inner products
+  // take 512 bytes per column
   std::vector<unsigned char> seen(std::max<int64_t>(n, 1), 0);
   bool blocked = !order.empty() && P.nnz < (int64_t)INT32_MAX && m < (int64_t)kCartNoRow &&
                  std::max(bits_for(m), 6) + bits_for((int64_t)(order.size() + kCartCols - 1) / kCartCols) <= 32;
   for (int j : order) {
-    blocked = blocked && !seen[j];
+    blocked = blocked && !seen[j] && std::isfinite(o.relaxpar / hn[j]);
     seen[j] = 1;
   }
   CartPlan &plan = P.cart_plan;
@@ -1111,7 +1113,9 @@ void run_cart(Problem &P, const airt_cart_opts &o, const double *d_b, const doub
   CartBlocks B{};
   size_t bsmem = 0;
   const bool rsmem = m <= kCartSharedRows;
-  DevBuf<double> od, xold, tail;
+  DevBuf<double> od, xold, rold, tail;
+  DevBuf<unsigned char> fold;
+  DevBuf<int> nfold;
   if (blocked && !st.stop) {
     if (replan) {
       build_plan(P, a, s);
@@ -1125,28 +1129,55 @@ void run_cart(Problem &P, const airt_cart_opts &o, const double *d_b, const doub
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(4 * kCartCols * kCartCols * sizeof(double) +
                                                kCartSharedRows * sizeof(double))));
+    xold.ensure(n);
+    rold.ensure(m);
     if (kmax >= o.kbegin) {  // some sweep may flag columns
-      xold.ensure(n);
+      fold.ensure(n);
+      nfold.ensure(n);
       tail.ensure(order.size());
       inorder.upload(seen.data(), n, s);
     }
   }
   int64_t l = 0;
+  auto copy = [&](auto *to, const auto *from, int64_t count) {
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(to, from, count * sizeof(*to), cudaMemcpyDeviceToDevice, s));
+  };
   for (int64_t k = 1; !st.stop; ++k) {
-    if (blocked) {
+    // The blocked sweep multiplies inner products with every step of a block,
+    // so an infinite or NaN step would reach columns that share no row with
+    // it (0 * NaN).  Such a step leaves its trace in the residual: a sweep
+    // that starts from or ends with a norm that is not finite is a general one.
+    bool finite = blocked && std::isfinite(resn.back());
+    double nrk = 0.0;
+    if (finite) {
       const bool flags = k >= o.kbegin;  // every flag is set before sweep kbegin
-      if (flags)
-        AIRT_CHECK_CUDA(cudaMemcpyAsync(xold.p, P.x64.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+      copy(xold.p, P.x64.p, n);
+      copy(rold.p, P.r64.p, m);
+      if (flags) {
+        copy(fold.p, flag.p, n);
+        copy(nfold.p, nflag.p, n);
+      }
       if (rsmem) k_cart_block<true><<<1, kCartBlockThreads, bsmem, s>>>(a, B);
       else k_cart_block<false><<<1, kCartBlockThreads, bsmem, s>>>(a, B);
       if (flags) k_cart_flags<<<1, 1024, 0, s>>>(a, k, xold.p, od.p, inorder.p, tail.p);
-    } else if (warp_sweep) {
-      k_cart_sweep_warp<<<1, 32, smem, s>>>(a, k);
-    } else {
-      k_cart_sweep_cta<<<1, kCartThreads, smem, s>>>(a, k);
+      AIRT_LAUNCH_CHECK();
+      nrk = judge_inputs(true);
+      finite = std::isfinite(nrk);
+      if (!finite) {
+        copy(P.x64.p, xold.p, n);
+        copy(P.r64.p, rold.p, m);
+        if (flags) {
+          copy(flag.p, fold.p, n);
+          copy(nflag.p, nfold.p, n);
+        }
+      }
     }
-    AIRT_LAUNCH_CHECK();
-    const double nrk = judge_inputs(true);
+    if (!finite) {
+      if (warp_sweep) k_cart_sweep_warp<<<1, 32, smem, s>>>(a, k);
+      else k_cart_sweep_cta<<<1, kCartThreads, smem, s>>>(a, k);
+      AIRT_LAUNCH_CHECK();
+      nrk = judge_inputs(true);
+    }
     resn.push_back(nrk);
     st.judge(k, nrk, ncc);
     if ((l < nK && k == K[l]) || st.stop) {
