@@ -79,15 +79,18 @@ __device__ __forceinline__ double par_sum(const ParGather &t, const RayGeom &g, 
     double d = fma(kd, t.D, t.s0) - c;
     if (qk.x > 0.0) {
       // at unit spacing two rays at most; without branches their loads and
-      // chords overlap
+      // chords overlap (a chord of 0 is no entry: u may not be finite there)
 #pragma unroll
       for (int q = 0; q < 2; ++q, ++k, d += t.D) {
         double uk = 0.0;
         if (d < wi.x && k < t.p) uk = u ? (double)__ldg(ua + k) : 1.0;
-        acc = fma(par_chord(wi.x, wi.y, qk.x, d), uk, acc);
+        const double chord = par_chord(wi.x, wi.y, qk.x, d);
+        acc = chord > 0.0 ? fma(chord, uk, acc) : acc;
       }
-      for (; d < wi.x && k < t.p; ++k, d += t.D)
-        acc = fma(par_chord(wi.x, wi.y, qk.x, d), u ? (double)__ldg(ua + k) : 1.0, acc);
+      for (; d < wi.x && k < t.p; ++k, d += t.D) {
+        const double chord = par_chord(wi.x, wi.y, qk.x, d);
+        if (chord > 0.0) acc = fma(chord, u ? (double)__ldg(ua + k) : 1.0, acc);
+      }
     } else {
       // axis-parallel: the pixel holds the rays whose coordinate floors to it
       const bool vert = cs.x != 0.0;  // rays along y at x = c*offset
