@@ -482,7 +482,10 @@ void par_prepare(Problem &P) {
   const double D = (off[P.p - 1] - off[0]) / (P.p - 1);
   // far finer rays than pixels would make a pixel's inner loop long
   if (!(D > 1.0 / 64) || !std::isfinite(D)) return;
-  const double tol = 8 * 2.2e-16 * std::fmax(std::fabs(off[0]), std::fabs(off[P.p - 1]));
+  // a few ulps of the offsets, but no more than shifts a chord by 1e-9 (a
+  // detector of 10^6 pixels or wider: its inner rays are finer than its ends)
+  const double tol =
+      std::fmin(8 * 2.2e-16 * std::fmax(std::fabs(off[0]), std::fabs(off[P.p - 1])), 1e-9);
   for (int k = 0; k < P.p; ++k)
     if (!(std::fabs(off[k] - (off[0] + k * D)) <= tol)) return;
   std::vector<ParAngle> t(P.nA);

@@ -1,4 +1,5 @@
-"""Pixel-driven back projection of values that are not finite."""
+"""Pixel-driven back projection at its edges: values that are not finite, and
+detectors far wider than the image."""
 import numpy as np
 import pytest
 
@@ -23,3 +24,19 @@ def test_values_that_are_not_finite_reach_their_own_pixels(theta, value):
         assert np.array_equal(np.isnan(want), np.isnan(got)) and np.array_equal(np.isinf(want), np.isinf(got))
         f = np.isfinite(want)
         assert np.all(np.abs(want[f] - got[f]) <= 2.0 ** -23 * np.abs(want[f]) + 1e-6)
+
+
+@pytest.mark.parametrize("d", [1e7 / 3, 1e13 / 3])
+@pytest.mark.parametrize("p", [7, 12])
+def test_wide_detectors(p, d):
+    """Offsets whose spacing rounds by more than a pixel's fraction; entries
+    agree to one FP32 step and 1e-8 of their crossings."""
+    N = 24
+    _, p, d, ct, st, off = T.parallel_tables(N, [0.0, 20.0, 45.0, 90.0, 118.0], p, d)
+    off = off + 3.3                                    # some rays through the image
+    S = T.parallel_operator(N, ct, st, off)
+    A = T.parallel_operator(N, ct, st, off, True)
+    u = np.random.default_rng(p).random(S.m)
+    a, b = S(u, "transp"), A(u, "transp")
+    assert np.all(np.abs(a - b) <= 2.0 ** -23 * np.abs(a) + 1e-8)
+    assert p % 2 == 0 or np.any(a > 0)
