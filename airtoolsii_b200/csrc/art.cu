@@ -381,6 +381,58 @@ uint64_t order_key(const int64_t *order, int64_t nsteps) {
   return h ? h : 1;
 }
 
+// Ranks of an order's entries on the device: two sorts' worth of work space,
+// 24-32 bytes per entry, for fewer than 2^32 entries.
+void rank_entries(Problem &P, const std::vector<int> &ord, const std::vector<int64_t> &toff, int64_t cnt, int64_t n,
+                  Schedule &S, cudaStream_t s) {
+  const int64_t nsteps = (int64_t)ord.size();
+  DevBuf<int> dord;
+  DevBuf<int64_t> dtoff;
+  DevBuf<unsigned> key, key2, at, at2, start;
+  DevBuf<unsigned char> tmp;
+  dord.upload(ord.data(), nsteps, s);
+  dtoff.upload(toff.data(), nsteps + 1, s);
+  key.ensure(cnt);
+  key2.ensure(cnt);
+  at.ensure(cnt);
+  at2.ensure(cnt);
+  start.ensure(n);
+  k_order_pixels<<<grid_for(nsteps * 32, 256), 256, 0, s>>>(nsteps, dord.p, dtoff.p, P.rp.p, P.ci.p, key.p, at.p);
+  AIRT_LAUNCH_CHECK();
+  int bits = 1;
+  while (bits < 31 && (1ll << bits) < n) ++bits;
+  size_t need = 0;
+  AIRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, need, key.p, key2.p, at.p, at2.p, cnt, 0, bits, s));
+  tmp.ensure(need);
+  AIRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, need, key.p, key2.p, at.p, at2.p, cnt, 0, bits, s));
+  const unsigned g = grid_for(cnt, 256);
+  k_run_starts<<<g, 256, 0, s>>>(cnt, key2.p, start.p);
+  k_ranks<<<g, 256, 0, s>>>(cnt, key2.p, at2.p, start.p, S.ent.p);
+  AIRT_LAUNCH_CHECK();
+}
+
+// The same on the host, where the device has no room for the sort or the
+// order visits more entries than it numbers; copied in slices.
+void rank_on_host(const std::vector<int64_t> &hrp, const std::vector<int> &hci, const std::vector<int> &ord,
+                  int64_t n, Schedule &S, cudaStream_t s) {
+  constexpr size_t kSlice = 4 << 20;
+  std::vector<unsigned> writes(n, 0);
+  std::vector<uint2> buf;
+  int64_t done = 0;
+  auto flush = [&] {
+    AIRT_CHECK_CUDA(cudaMemcpyAsync(S.ent.p + done, buf.data(), buf.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
+    AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+    done += (int64_t)buf.size();
+    buf.clear();
+  };
+  for (const int row : ord)
+    for (int64_t e = hrp[row]; e < hrp[row + 1]; ++e) {
+      buf.push_back(make_uint2((unsigned)hci[e], writes[hci[e]]++));
+      if (buf.size() == kSlice) flush();
+    }
+  flush();
+}
+
 // Level schedule of a row order (see the file comment): the levels on the
 // host, the entries' ranks on the device.
 void build_schedule(Problem &P, const std::vector<int64_t> &hrp, const std::vector<int> &hci,
@@ -409,7 +461,6 @@ void build_schedule(Problem &P, const std::vector<int64_t> &hrp, const std::vect
   S.nlev = maxlev + 1;
   S.nsteps = nsteps;
   const int64_t cnt = toff[nsteps];
-  AIRT_REQUIRE(cnt < (int64_t)UINT32_MAX, "the row order visits too many entries");
   std::vector<int> ptr(S.nlev + 1, 0);
   std::vector<ArtStep> steps(nsteps);
   for (int64_t t = 0; t < nsteps; ++t) ++ptr[level[t] + 1];
@@ -421,31 +472,16 @@ void build_schedule(Problem &P, const std::vector<int64_t> &hrp, const std::vect
   }
   S.steps.upload(steps.data(), nsteps, s);
   S.ent.ensure(cnt);
-  if (cnt) {
-    DevBuf<int> dord;
-    DevBuf<int64_t> dtoff;
-    DevBuf<unsigned> key, key2, at, at2, start;
-    DevBuf<unsigned char> tmp;
-    dord.upload(ord.data(), nsteps, s);
-    dtoff.upload(toff.data(), nsteps + 1, s);
-    key.ensure(cnt);
-    key2.ensure(cnt);
-    at.ensure(cnt);
-    at2.ensure(cnt);
-    start.ensure(n);
-    k_order_pixels<<<grid_for(nsteps * 32, 256), 256, 0, s>>>(nsteps, dord.p, dtoff.p, P.rp.p, P.ci.p, key.p, at.p);
-    AIRT_LAUNCH_CHECK();
-    int bits = 1;
-    while (bits < 31 && (1ll << bits) < n) ++bits;
-    size_t need = 0;
-    AIRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, need, key.p, key2.p, at.p, at2.p, cnt, 0, bits, s));
-    tmp.ensure(need);
-    AIRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, need, key.p, key2.p, at.p, at2.p, cnt, 0, bits, s));
-    const unsigned g = grid_for(cnt, 256);
-    k_run_starts<<<g, 256, 0, s>>>(cnt, key2.p, start.p);
-    k_ranks<<<g, 256, 0, s>>>(cnt, key2.p, at2.p, start.p, S.ent.p);
-    AIRT_LAUNCH_CHECK();
+  bool ranked = cnt == 0;
+  if (!ranked && cnt < (int64_t)UINT32_MAX) {
+    try {
+      rank_entries(P, ord, toff, cnt, n, S, s);
+      ranked = true;
+    } catch (const Status &e) {
+      if (e.code != AIRT_ERR_OOM) throw;
+    }
   }
+  if (!ranked) rank_on_host(hrp, hci, ord, n, S, s);
   AIRT_CHECK_CUDA(cudaStreamSynchronize(s));  // the host vectors and work space end here
 }
 
