@@ -1116,11 +1116,20 @@ void run_cart(Problem &P, const airt_cart_opts &o, const double *d_b, const doub
   DevBuf<double> od, xold, rold, tail;
   DevBuf<unsigned char> fold;
   DevBuf<int> nfold;
-  if (blocked && !st.stop) {
-    if (replan) {
+  if (replan && !st.stop) {
+    try {
       build_plan(P, a, s);
       plan.key = key;
+    } catch (const Status &e) {
+      if (e.code != AIRT_ERR_OOM) throw;
+      // no room for the inner products: the general sweep needs none
+      plan.cbase.release();
+      plan.ent.release();
+      plan.gram.release();
+      blocked = false;
     }
+  }
+  if (blocked && !st.stop) {
     od.ensure(order.size());
     B = CartBlocks{plan.nblocks, plan.cbase.p, plan.ent.p, plan.gram.p, od.p};
     bsmem = 4 * kCartCols * kCartCols * sizeof(double) + (rsmem ? (size_t)m * sizeof(double) : 0);

@@ -1,6 +1,7 @@
-"""Row sweeps when the device has no room for their schedule's work space: the
-call goes on without it.  Allocations fail one after the other by the
-host-side hook.  Tolerance: the suite's bar for ART, 1e-5."""
+"""Row and column sweeps when the device has no room for their schedules' work
+space: the call goes on without it.  Allocations fail one after the other by
+the host-side hook.  Tolerances: the suite's bars for ART (1e-5) and CART (1e-9
+on the FP32-rounded matrix)."""
 import numpy as np
 import pytest
 
@@ -40,3 +41,12 @@ def test_kaczmarz_ranks_on_the_host(method):
     want = O.art(method, M, b, [4])[0][:, -1]
     out = outcomes(lambda A: getattr(airt, method)(A, b, [4])[0][:, -1], want, 1e-5)
     assert "ok" in out[:len(out) - out[::-1].index("oom")]     # one that failed before the last that must not
+
+
+def test_cart_without_a_plan():
+    M = O.paralleltomo_matrix(20, TH).tocsc()
+    M.data = M.data.astype(np.float32).astype(np.float64)
+    b = M @ O.shepplogan(20)
+    want = O.cart("columnaction", M, b, [4])[0][:, -1]
+    out = outcomes(lambda A: airt.columnaction(A, b, [4])[0][:, -1], want, 1e-9)
+    assert "ok" in out[:len(out) - out[::-1].index("oom")]
