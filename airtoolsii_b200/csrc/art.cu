@@ -371,16 +371,6 @@ __global__ void k_copy_d(int64_t n, const double *__restrict__ a, double *__rest
 
 using Schedule = ArtSchedule;
 
-// FNV-1a hash of a row order (the key of the cached schedule; never 0).
-uint64_t order_key(const int64_t *order, int64_t nsteps) {
-  uint64_t h = 1469598103934665603ull ^ (uint64_t)nsteps;
-  for (int64_t t = 0; t < nsteps; ++t) {
-    h ^= (uint64_t)order[t];
-    h *= 1099511628211ull;
-  }
-  return h ? h : 1;
-}
-
 // Ranks of an order's entries on the device: two sorts' worth of work space,
 // 24-32 bytes per entry, for fewer than 2^32 entries.
 void rank_entries(Problem &P, const std::vector<int> &ord, const std::vector<int64_t> &toff, int64_t cnt, int64_t n,
@@ -562,8 +552,8 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
   const bool per_sweep_sched = (o.order_kind == 2 && stride > 0);
   Schedule local;
   Schedule &S = per_sweep_sched ? local : P.art_sched;
-  const uint64_t key = per_sweep_sched ? 0 : order_key(order.data(), per_sweep);
-  const bool need_pattern = per_sweep_sched || S.key != key || S.nsteps != per_sweep;
+  const bool need_pattern = per_sweep_sched || !S.ready || (int64_t)S.order.size() != per_sweep ||
+                            !std::equal(S.order.begin(), S.order.end(), order.begin());
   // host copy of the sparsity pattern, only when a schedule is built
   std::vector<int64_t> hrp;
   std::vector<int> hci;
@@ -577,9 +567,10 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
     AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
   }
   if (!per_sweep_sched && need_pattern) {
-    S.key = 0;
+    S.ready = false;
     build_schedule(P, hrp, hci, order.data(), per_sweep, n, S, s);
-    S.key = key;
+    S.order.assign(order.begin(), order.begin() + per_sweep);
+    S.ready = true;
   }
 
   // iterate

@@ -859,16 +859,6 @@ __global__ void k_sumsq(int64_t m, const double *__restrict__ r, double *__restr
   if (threadIdx.x == 0) atomicAdd(out, v);
 }
 
-// FNV-1a hash of a column order (the key of the plan; never 0).
-uint64_t cols_key(const std::vector<int> &order) {
-  uint64_t h = 1469598103934665603ull ^ (uint64_t)order.size();
-  for (int j : order) {
-    h ^= (uint64_t)(unsigned)j;
-    h *= 1099511628211ull;
-  }
-  return h ? h : 1;
-}
-
 int bits_for(int64_t count) {  // bits that hold 0..count-1
   int b = 1;
   while (b < 62 && (1ll << b) < count) ++b;
@@ -1006,13 +996,12 @@ void run_cart(Problem &P, const airt_cart_opts &o, const double *d_b, const doub
     seen[j] = 1;
   }
   CartPlan &plan = P.cart_plan;
-  const uint64_t key = blocked ? cols_key(order) : 0;
-  const bool replan = blocked && plan.key != key;
+  const bool replan = blocked && !(plan.ready && plan.order == order);
   DevBuf<int> own_cols, nflag, err;
   DevBuf<int> &cols = blocked ? plan.cols : own_cols;
   DevBuf<unsigned char> flag, inorder;
   if (!blocked || replan) {
-    plan.key = blocked ? 0 : plan.key;
+    if (blocked) plan.ready = false;
     cols.upload(order.data(), order.size(), s);
   }
   nflag.ensure(std::max<int64_t>(n, 1));
@@ -1119,7 +1108,8 @@ void run_cart(Problem &P, const airt_cart_opts &o, const double *d_b, const doub
   if (replan && !st.stop) {
     try {
       build_plan(P, a, s);
-      plan.key = key;
+      plan.order = order;
+      plan.ready = true;
     } catch (const Status &e) {
       if (e.code != AIRT_ERR_OOM) throw;
       // no room for the inner products: the general sweep needs none

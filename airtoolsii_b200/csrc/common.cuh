@@ -198,7 +198,8 @@ struct ArtStep {
 struct ArtSchedule {
   int nlev = 0;
   int64_t nsteps = 0;
-  uint64_t key = 0;  // hash of the row order it was built for (0: none)
+  bool ready = false;
+  std::vector<int64_t> order;  // the row order it was built for
   DevBuf<ArtStep> steps;
   DevBuf<uint2> ent;
 };
@@ -208,8 +209,9 @@ struct ArtSchedule {
 // entries of a block sorted by row, and the columns' inner products.
 struct CartPlan {
   int64_t nblocks = 0;
-  uint64_t key = 0;  // hash of the column order it was built for (0: none)
-  DevBuf<int> cols;              // the order
+  bool ready = false;
+  std::vector<int> order;        // the column order it was built for
+  DevBuf<int> cols;              // the same on the device
   DevBuf<int64_t> cbase;         // nblocks + 1 offsets into the chunks
   DevBuf<uint2> ent;             // chunks of 32 sorted entries: row | column of the block << 27, value bits
   DevBuf<double> gram;           // nblocks x 2*kCartCols x kCartCols
