@@ -452,16 +452,4 @@ __device__ __forceinline__ void row_entries(const RayGeom &g, int64_t r, bool ex
   trace_entries(g.N, ray_of(g, r), exclude_top_right, emit);
 }
 
-// row_entries for one of the two threads that share row r (part 0 or 1):
-// straight rays are split by trace_entries_part; a circle goes to part 0.
-template <class Emit>
-__device__ __forceinline__ void row_entries_part(const RayGeom &g, int64_t r, bool exclude_top_right, int part,
-                                                 Emit &&emit) {
-  if (g.kind == GEO_SPHERE) {
-    if (part == 0) row_entries(g, r, exclude_top_right, emit);
-    return;
-  }
-  trace_entries_part(g.N, ray_of(g, r), exclude_top_right, part, emit);
-}
-
 }  // namespace airt
