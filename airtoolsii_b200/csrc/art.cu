@@ -81,11 +81,15 @@ __device__ __forceinline__ double clamp_scalar(double v, const KaczArgs &a) {
   return a.ubk != AIRT_BOUND_NONE && !(v <= a.ub) ? a.ub : v;
 }
 
-// Test hook: a cycle budget for the bounded waits of the sweep kernel and
-// an injected stall (the first step waits for a stamp that no step writes),
-// so that a test can make a wait run out.  Defaults: ~2 s, no stall.
-long long g_kacz_wait_budget = 4000000000ll;
-int g_kacz_inject_stall = 0;
+}  // namespace
+
+// Cycle budget of the bounded waits (the sweep's, and the grid barriers of
+// persist.cuh; ~2 s), and a test hook that makes a wait run out: the first
+// step waits for a stamp that no step writes, a barrier for an arrival more.
+long long g_wait_budget = 4000000000ll;
+int g_inject_stall = 0;
+
+namespace {
 
 constexpr int kDagThreads = 256;  // eight warps per CTA
 
@@ -590,8 +594,8 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
   AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kacz_sweep, kDagThreads, 0));
   AIRT_REQUIRE(occ >= 1, "the Kaczmarz sweep kernel cannot be resident");
   const int dag_grid = num_sms();
-  const long long budget = g_kacz_wait_budget;
-  const int stall = g_kacz_inject_stall;
+  const long long budget = g_wait_budget;
+  const int stall = g_inject_stall;
   int herr = 0;
   DevBuf<double> tab, red, keep;
   if (o.relax_table && kmax > 0) tab.upload(o.relax_table, kmax * per_sweep, s);
@@ -721,11 +725,11 @@ void run_art(Problem &P, const airt_art_opts &o, const double *d_b, const double
 
 extern "C" int airt_test_set_wait_budget(long long cycles) {
   if (cycles <= 0) return AIRT_ERR_ARG;
-  airt::g_kacz_wait_budget = cycles;
+  airt::g_wait_budget = cycles;
   return AIRT_OK;
 }
 
 extern "C" int airt_test_inject_stall(int on) {
-  airt::g_kacz_inject_stall = on ? 1 : 0;
+  airt::g_inject_stall = on ? 1 : 0;
   return AIRT_OK;
 }

@@ -586,6 +586,7 @@ struct TailArgs {
   unsigned *counter;
   int *err;
   long long budget;
+  unsigned stall;  // test hook: barriers wait for one arrival more than there is
   int64_t kmax;
 };
 
@@ -642,7 +643,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_batch_tail(const __grid_con
   for (int q = threadIdx.x; q < a.cols.p0[kClasses]; q += kTailThreads) pc[q] = a.cols.pieces[q];
   unsigned target = 0;
   auto barrier = [&]() {
-    return persist_barrier(a.counter, target += gridDim.x, a.err, a.budget, [] {});
+    return persist_barrier(a.counter, (target += gridDim.x) + a.stall, a.err, a.budget, [] {});
   };
   // which instances run on; false when none does
   auto look = [&]() -> bool {
@@ -1318,7 +1319,8 @@ bool batch_tail(Batch &B, const BFwd &fo, const BUpd &uo, const BCtrl &co, int64
   AIRT_CHECK_CUDA(cudaMemsetAsync(P.err.p, 0, sizeof(int), s));
   a.counter = B.tail_count.p;
   a.err = P.err.p;
-  a.budget = kPersistWaitBudget;
+  a.budget = g_wait_budget;
+  a.stall = (unsigned)g_inject_stall;
   a.kmax = kmax;
   constexpr int64_t kIters = 2048;  // per launch
   for (int64_t it = done; it < kmax;) {

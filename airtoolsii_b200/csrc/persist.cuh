@@ -22,8 +22,9 @@
 
 namespace airt {
 
-// Cycle budget of a barrier wait (~2 s).
-constexpr long long kPersistWaitBudget = 4000000000ll;
+// Cycle budget of a wait, and the test hook that makes one run out (art.cu).
+extern long long g_wait_budget;
+extern int g_inject_stall;
 
 // One direction of the matrix: segments ptr[i]..ptr[i+1] of idx and val, L
 // lanes per segment.

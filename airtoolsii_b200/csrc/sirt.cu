@@ -423,6 +423,7 @@ struct PersistArgs {
   unsigned *count;   // barrier counter, zeroed before the launch
   int *err;
   long long budget;
+  unsigned stall;    // test hook: barriers wait for one arrival more than there is
   int it0, it1;
 };
 
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_sirt_persist(const __grid_consta
     }
     r2 = warp_sum(r2);
     if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = r2;
-    return persist_barrier(a.count, target += gridDim.x, a.err, a.budget, [&] {
+    return persist_barrier(a.count, (target += gridDim.x) + a.stall, a.err, a.budget, [&] {
       double v = 0.0;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) v += sums[w];
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_sirt_persist(const __grid_consta
       const double g = persist_group_sum(persist_dot_again<kAhead>(a.cols, j, lc, a.mr32), a.cols.L);
       if (lc == 0 && j < a.cols.nseg) update_x_pre(j, g, lam, a.u, slot, a.u.x64[j], a.u.D[j]);
     }
-    if (!persist_barrier(a.count, target += gridDim.x, a.err, a.budget, [] {})) return;
+    if (!persist_barrier(a.count, (target += gridDim.x) + a.stall, a.err, a.budget, [] {})) return;
     if (!forward(it)) return;
   }
 }
@@ -819,7 +820,8 @@ void run_persist(Problem &P, const FwdOut &fo, const UpdArgs &ua, int64_t kmax) 
   a.part = P.pst_part.p;
   a.count = P.pst_count.p;
   a.err = P.err.p;
-  a.budget = kPersistWaitBudget;
+  a.budget = g_wait_budget;
+  a.stall = (unsigned)g_inject_stall;
   ensure_h_state(P);
   for (int64_t it = 0; it < kmax; it = a.it1) {
     a.it0 = (int)it;

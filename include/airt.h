@@ -389,10 +389,12 @@ int airt_release_memory(void);
 /* ---- test hooks ----------------------------------------------------------- */
 /* No counterpart in the reference.  For tests of the bounded device waits:
  * airt_test_set_wait_budget sets the clock64 cycle budget of each wait of the
- * Kaczmarz sweep kernel (default 4e9, about 2 s); airt_test_inject_stall(1)
- * makes the first step of every sweep wait for a completion stamp that no
- * step writes, so the wait runs out, the kernel leaves and airt_art returns
- * AIRT_ERR_TIMEOUT.  Process-wide; not for production use. */
+ * Kaczmarz sweep kernel and of the grid barriers of the one-launch SIRT and
+ * batch kernels (default 4e9, about 2 s).  airt_test_inject_stall(1) makes the
+ * first step of every sweep wait for a completion stamp that no step writes,
+ * and every grid barrier for one arrival more than there is, so the wait runs
+ * out, the kernel leaves and the call returns AIRT_ERR_TIMEOUT.  Process-wide;
+ * not for production use. */
 int airt_test_set_wait_budget(long long cycles);
 int airt_test_inject_stall(int on);
 /* airt_test_fail_alloc(k), k >= 0: the next k device allocations of the
