@@ -4,13 +4,20 @@
 // two launches and, in each product, the chain row pointer -> entries ->
 // gather -> sum (12 us per iteration at N = 64, 30 angles, where the bytes
 // take less than 1 us).  Here one CTA per SM stays for the whole solve.  A
-// group of lanes owns the same rows and columns in every iteration and keeps
-// the first kResident 16-byte vectors of its first segment per lane (values
-// and indices, both directions) in registers, so that of the chain only the
-// gather and the sum remain between two grid barriers; what does not fit is
-// read from L2 again.  The stopping rule needs no launch either: every CTA
-// adds the CTAs' partial sums in the same order and takes the same decision
-// while the gathers of the next update are in flight.
+// group of threads owns the same rows and columns in every iteration and keeps
+// the first entries of its first segment per thread (values and indices, both
+// directions) in registers, so that of the chain only the gather and the sum
+// remain between two grid barriers; what does not fit is read from L2 again.
+// The stopping rule needs no launch either: every CTA adds the CTAs' partial
+// sums in the same order and takes the same decision while the gathers of the
+// next update are in flight.
+//
+// Every sum is taken in the order of the launched kernels
+// (for_each_segment_vpre of spmv.cuh): L lanes per segment, four accumulators
+// per lane, one for each element of the 16-byte vectors.  An FP64 sum in
+// another order differs in its last bit, which flips the FP32 rounding of x or
+// M.*r now and then: 5e-10 of x after 1,500 iterations.  More threads than L
+// lanes come from the accumulators: C of the four per thread.
 //
 // The grid barrier is a counter that every CTA raises and waits on; the
 // launch is cooperative, so all CTAs are resident.  Each wait is bounded: on
@@ -19,6 +26,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "spmv.cuh"
 
 namespace airt {
 
@@ -26,77 +34,90 @@ namespace airt {
 extern long long g_wait_budget;
 extern int g_inject_stall;
 
-// One direction of the matrix: segments ptr[i]..ptr[i+1] of idx and val, L
-// lanes per segment.
+// One direction of the matrix: segments ptr[i]..ptr[i+1] of idx and val (fewer
+// than 2^30 of them and of nonzeros), L lanes of S threads per segment; thread
+// `sub` of a lane has the accumulators of the vector elements sub*C .. sub*C + C-1.
 struct PersistDir {
   int nseg;
   const int64_t *ptr;
   const int *idx;
   const float *val;
-  int L;
+  int L, C, S, T;  // S = 4 / C, T = L * S threads per segment
 };
 
-// Lanes per segment for `threads` threads: the fewest vector loads in a row per
-// lane, where a segment's fixed part (bounds, reduction, epilogue) counts as
-// three.
-inline int persist_lanes(int64_t nnz, int64_t nseg, int64_t threads) {
-  const double avg = nseg ? (double)nnz / (double)nseg : 0.0;
-  int best = 2;
+// The split for `threads` threads: L as the launched kernels have it, and the
+// C with the fewest vectors' worth of loads in a row per thread, where a
+// segment's fixed part (bounds, reduction, epilogue) counts as three.
+inline void persist_split(PersistDir &d, int64_t nnz, int64_t threads) {
+  const double avg = d.nseg ? (double)nnz / (double)d.nseg : 0.0;
+  d.L = vec_lanes_for(nnz, d.nseg);
   double cost = INFINITY;
-  for (int L = 2; L <= 32; L *= 2) {
-    const double c = std::ceil((double)nseg * L / (double)threads) * (avg / (4.0 * L) + 3.0);
-    if (c < cost) {
-      cost = c;
-      best = L;
-    }
+  for (int C = 4; C >= 1; C /= 2) {
+    const int T = d.L * 4 / C;
+    const double c = std::ceil((double)d.nseg * T / (double)threads) * (avg / (4.0 * T) + 3.0);
+    if (c >= cost) continue;
+    cost = c;
+    d.C = C;
+    d.S = 4 / C;
+    d.T = T;
   }
-  return best;
 }
 
-// The resident part of a lane's first segment: vectors v, v + L, ... of the
-// aligned groups that overlap it, a mask bit per element inside the segment,
-// and where the rest of the segment's vectors starts.
-template <int R>
-struct PersistSeg {
-  float4 f[R > 0 ? R : 1];
-  int4 c[R > 0 ? R : 1];
-  unsigned mask;
-  int v, ve;     // next vector of this lane and end, relative to base
-  int64_t base;  // first vector of the segment
-  int lo, hi;    // first and last + 1 element of the segment, relative to 4*base
+// Where a thread's part of a segment lies: nonzeros [q0, q1), whole vectors
+// [qa, qb) of them; the others are added first, those before qa to the first
+// accumulator, those from qb on to the second.
+struct PersistPart {
+  int q0, q1, qa, qb, lane, sub;
 };
 
-template <int R>
-__device__ __forceinline__ PersistSeg<R> persist_load(const PersistDir &d, int seg, int lane) {
-  PersistSeg<R> s;
-  s.mask = 0;
-  int64_t q0 = 0, q1 = 0;
+__device__ __forceinline__ PersistPart persist_part(const PersistDir &d, int seg, int t) {
+  PersistPart p{0, 0, 0, 0, t / d.S, t % d.S};
   if (seg < d.nseg) {
-    q0 = __ldg(d.ptr + seg);
-    q1 = __ldg(d.ptr + seg + 1);
+    p.q0 = (int)__ldg(d.ptr + seg);
+    p.q1 = (int)__ldg(d.ptr + seg + 1);
   }
-  s.base = q0 >> 2;
-  s.lo = (int)(q0 - 4 * s.base);
-  s.hi = (int)(q1 - 4 * s.base);
-  s.ve = q1 > q0 ? (s.hi + 3) >> 2 : 0;
+  p.qa = min((p.q0 + 3) & ~3, p.q1);
+  p.qb = max(p.q1 & ~3, p.qa);
+  return p;
+}
+
+// The resident part of a thread's first segment (L > 2, so that a thread has
+// at most one element before the whole vectors and one after them): the
+// element before, the one after, the first R of the vectors', and where the
+// rest starts.
+template <int C, int R>
+struct PersistSeg {
+  float f[R > 0 ? R : 1], fe[2];
+  int c[R > 0 ? R : 1], ce[2];
+  int have;    // whole vectors held
+  bool on[2];  // the element before, the one after
+  int v, ve;   // next vector of this lane and end
+  int sub;
+};
+
+template <int C, int R>
+__device__ __forceinline__ PersistSeg<C, R> persist_load(const PersistDir &d, int seg, int t) {
+  const PersistPart p = persist_part(d, seg, t);
+  PersistSeg<C, R> s;
+  s.sub = p.sub;
+  const int h = p.q0 + p.lane, g = p.qb + p.lane;
+  s.on[0] = p.sub == 0 && h < p.qa;
+  s.on[1] = p.sub == (C == 1 ? 1 : 0) && g < p.q1;
 #pragma unroll
-  for (int u = 0; u < R; ++u) {
-    const int v = lane + u * d.L;
-    s.f[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    s.c[u] = make_int4(0, 0, 0, 0);
-    if (v < s.ve) {
-      s.f[u] = __ldg(reinterpret_cast<const float4 *>(d.val) + s.base + v);
-      const int4 c = __ldg(reinterpret_cast<const int4 *>(d.idx) + s.base + v);
-      const int e = 4 * v;
-      unsigned k = 0;
-      if (e >= s.lo && e < s.hi) { k |= 1u; s.c[u].x = c.x; }
-      if (e + 1 >= s.lo && e + 1 < s.hi) { k |= 2u; s.c[u].y = c.y; }
-      if (e + 2 >= s.lo && e + 2 < s.hi) { k |= 4u; s.c[u].z = c.z; }
-      if (e + 3 >= s.lo && e + 3 < s.hi) { k |= 8u; s.c[u].w = c.w; }
-      s.mask |= k << (4 * u);
-    }
+  for (int i = 0; i < 2; ++i) {
+    s.fe[i] = s.on[i] ? __ldg(d.val + (i ? g : h)) : 0.f;
+    s.ce[i] = s.on[i] ? __ldg(d.idx + (i ? g : h)) : 0;
   }
-  s.v = lane + R * d.L;
+  const int v0 = (p.qa >> 2) + p.lane;
+  s.ve = p.qb >> 2;
+  s.have = min(R / C, max(0, (s.ve - v0 + d.L - 1) / d.L));
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int u = i / C, q = 4 * (v0 + u * d.L) + p.sub * C + i % C;
+    s.f[i] = u < s.have ? __ldg(d.val + q) : 0.f;
+    s.c[i] = u < s.have ? __ldg(d.idx + q) : 0;
+  }
+  s.v = v0 + R / C * d.L;
   return s;
 }
 
@@ -112,92 +133,110 @@ __device__ __forceinline__ int fresh(int v) {
   return v;
 }
 
-// Sum over the lane's own elements of a resident segment; x is written by
-// other CTAs between barriers, so it is read with plain loads.
-template <int R>
-__device__ __forceinline__ double persist_dot(const PersistDir &d, const PersistSeg<R> &s, const float *x) {
-  float4 g[R > 0 ? R : 1];
-#pragma unroll
-  for (int u = 0; u < R; ++u)
-    if (s.mask >> (4 * u) & 15u) g[u] = make_float4(x[fresh(s.c[u].x)], x[fresh(s.c[u].y)], x[fresh(s.c[u].z)], x[fresh(s.c[u].w)]);
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-#pragma unroll
-  for (int u = 0; u < R; ++u) {
-    if (s.mask >> (4 * u) & 1u) a0 = fma((double)fresh(s.f[u].x), (double)g[u].x, a0);
-    if (s.mask >> (4 * u) & 2u) a1 = fma((double)fresh(s.f[u].y), (double)g[u].y, a1);
-    if (s.mask >> (4 * u) & 4u) a2 = fma((double)fresh(s.f[u].z), (double)g[u].z, a2);
-    if (s.mask >> (4 * u) & 8u) a3 = fma((double)fresh(s.f[u].w), (double)g[u].w, a3);
-  }
+// Adds vectors v, v + L, .. < ve of the thread's C accumulators to a[0..C),
+// AHEAD vectors in flight; x is written by other CTAs between barriers, so it
+// is read with plain loads.
+template <int C, int AHEAD>
+__device__ __forceinline__ void persist_vectors(const PersistDir &d, int v, int ve, int sub, const float *x,
+                                                double *a) {
+  auto load = [&](int w, float *f, int *c) {
+    const float *fp = d.val + 4 * w + sub * C;
+    const int *cp = d.idx + 4 * w + sub * C;
+    if (C == 4) {
+      const float4 f4 = __ldg(reinterpret_cast<const float4 *>(fp));
+      const int4 c4 = __ldg(reinterpret_cast<const int4 *>(cp));
+      f[0] = f4.x, f[1] = f4.y, f[2] = f4.z, f[3] = f4.w;
+      c[0] = c4.x, c[1] = c4.y, c[2] = c4.z, c[3] = c4.w;
+    } else if (C == 2) {
+      const float2 f2 = __ldg(reinterpret_cast<const float2 *>(fp));
+      const int2 c2 = __ldg(reinterpret_cast<const int2 *>(cp));
+      f[0] = f2.x, f[1] = f2.y;
+      c[0] = c2.x, c[1] = c2.y;
+    } else {
+      f[0] = __ldg(fp);
+      c[0] = __ldg(cp);
+    }
+  };
 #pragma unroll 1
-  for (int v = s.v; v < s.ve; v += d.L) {
-    const float4 f = __ldg(reinterpret_cast<const float4 *>(d.val) + s.base + v);
-    const int4 c = __ldg(reinterpret_cast<const int4 *>(d.idx) + s.base + v);
-    const int e = 4 * v;  // v > 0, so only the segment's end can cut the vector
-    a0 = fma((double)f.x, (double)x[c.x], a0);
-    if (e + 1 < s.hi) a1 = fma((double)f.y, (double)x[c.y], a1);
-    if (e + 2 < s.hi) a2 = fma((double)f.z, (double)x[c.z], a2);
-    if (e + 3 < s.hi) a3 = fma((double)f.w, (double)x[c.w], a3);
+  for (; v + (AHEAD - 1) * d.L < ve; v += AHEAD * d.L) {
+    float f[AHEAD][C], g[AHEAD][C];
+    int c[AHEAD][C];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) load(v + u * d.L, f[u], c[u]);
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+      for (int k = 0; k < C; ++k) g[u][k] = x[c[u][k]];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+      for (int k = 0; k < C; ++k) a[k] = fma((double)f[u][k], (double)g[u][k], a[k]);
   }
-  return (a0 + a1) + (a2 + a3);
+  if (AHEAD > 1)
+#pragma unroll 1
+    for (; v < ve; v += d.L) {
+      float f[C];
+      int c[C];
+      load(v, f, c);
+#pragma unroll
+      for (int k = 0; k < C; ++k) a[k] = fma((double)f[k], (double)x[c[k]], a[k]);
+    }
+}
+
+template <int C>
+__device__ __forceinline__ double persist_fold(const double *a) {
+  return C == 4 ? (a[0] + a[1 % C]) + (a[2 % C] + a[3 % C]) : C == 2 ? a[0] + a[1 % C] : a[0];
+}
+
+// The thread's part of the sum over a resident segment.
+template <int C, int R>
+__device__ __forceinline__ double persist_dot(const PersistDir &d, const PersistSeg<C, R> &s, const float *x) {
+  float g[R > 0 ? R : 1], ge[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (s.on[i]) ge[i] = x[fresh(s.ce[i])];
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+    if (i / C < s.have) g[i] = x[fresh(s.c[i])];
+  double a[C] = {};
+  if (s.on[0]) a[0] = fma((double)fresh(s.fe[0]), (double)ge[0], a[0]);
+  if (s.on[1]) a[1 % C] = fma((double)fresh(s.fe[1]), (double)ge[1], a[1 % C]);
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+    if (i / C < s.have) a[i % C] = fma((double)fresh(s.f[i]), (double)g[i], a[i % C]);
+  persist_vectors<C, 1>(d, s.v, s.ve, s.sub, x, a);
+  return persist_fold<C>(a);
 }
 
 // The same for a segment that is read again in every iteration.
-template <int AHEAD>
-__device__ __forceinline__ double persist_dot_again(const PersistDir &d, int seg, int lane, const float *x) {
-  int64_t q0 = 0, q1 = 0;
-  if (seg < d.nseg) {
-    q0 = __ldg(d.ptr + seg);
-    q1 = __ldg(d.ptr + seg + 1);
-  }
-  const int64_t ve = q1 > q0 ? (q1 + 3) >> 2 : 0;
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-  auto masked = [&](int64_t v) {
-    const float4 f = __ldg(reinterpret_cast<const float4 *>(d.val) + v);
-    const int4 c = __ldg(reinterpret_cast<const int4 *>(d.idx) + v);
-    const int64_t e = v << 2;
-    if (e >= q0 && e < q1) a0 = fma((double)f.x, (double)x[c.x], a0);
-    if (e + 1 >= q0 && e + 1 < q1) a1 = fma((double)f.y, (double)x[c.y], a1);
-    if (e + 2 >= q0 && e + 2 < q1) a2 = fma((double)f.z, (double)x[c.z], a2);
-    if (e + 3 >= q0 && e + 3 < q1) a3 = fma((double)f.w, (double)x[c.w], a3);
-  };
-  // the vectors cut by the segment's ends, then the others AHEAD at a time
-  const int64_t vb = (q0 + 3) >> 2, vl = q1 >> 2;
-  if (lane == 0 && vb > (q0 >> 2) && q1 > q0) masked(q0 >> 2);
-  if (lane == d.L - 1 && vl >= vb && ve > vl) masked(vl);
-  int64_t v = vb + lane;
-  for (; v + (AHEAD - 1) * d.L < vl; v += AHEAD * d.L) {
-    float4 f[AHEAD];
-    int4 c[AHEAD];
-#pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      f[u] = __ldg(reinterpret_cast<const float4 *>(d.val) + v + u * d.L);
-      c[u] = __ldg(reinterpret_cast<const int4 *>(d.idx) + v + u * d.L);
+template <int C, int AHEAD>
+__device__ __forceinline__ double persist_again_c(const PersistDir &d, const PersistPart &p, const float *x) {
+  double a[C] = {};
+  if (p.sub == 0)
+    for (int q = p.q0 + p.lane; q < p.qa; q += d.L) a[0] = fma((double)__ldg(d.val + q), (double)x[__ldg(d.idx + q)], a[0]);
+  if (p.sub == (C == 1 ? 1 : 0))
+    for (int q = p.qb + p.lane; q < p.q1; q += d.L) {
+      double &t = a[C > 1 ? 1 % C : 0];
+      t = fma((double)__ldg(d.val + q), (double)x[__ldg(d.idx + q)], t);
     }
-    float4 g[AHEAD];
-#pragma unroll
-    for (int u = 0; u < AHEAD; ++u) g[u] = make_float4(x[c[u].x], x[c[u].y], x[c[u].z], x[c[u].w]);
-#pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      a0 = fma((double)f[u].x, (double)g[u].x, a0);
-      a1 = fma((double)f[u].y, (double)g[u].y, a1);
-      a2 = fma((double)f[u].z, (double)g[u].z, a2);
-      a3 = fma((double)f[u].w, (double)g[u].w, a3);
-    }
-  }
-#pragma unroll 1
-  for (; v < vl; v += d.L) {
-    const float4 f = __ldg(reinterpret_cast<const float4 *>(d.val) + v);
-    const int4 c = __ldg(reinterpret_cast<const int4 *>(d.idx) + v);
-    a0 = fma((double)f.x, (double)x[c.x], a0);
-    a1 = fma((double)f.y, (double)x[c.y], a1);
-    a2 = fma((double)f.z, (double)x[c.z], a2);
-    a3 = fma((double)f.w, (double)x[c.w], a3);
-  }
-  return (a0 + a1) + (a2 + a3);
+  persist_vectors<C, AHEAD>(d, (p.qa >> 2) + p.lane, p.qb >> 2, p.sub, x, a);
+  return persist_fold<C>(a);
 }
 
-__device__ __forceinline__ double persist_group_sum(double v, int L) {
-  for (int o = L >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// K: the direction's C, or 0 where the kernel is made for any.
+template <int K, int AHEAD>
+__device__ __forceinline__ double persist_dot_again(const PersistDir &d, int seg, int t, const float *x) {
+  const PersistPart p = persist_part(d, seg, t);
+  if (K) return persist_again_c<K ? K : 1, AHEAD>(d, p, x);
+  return d.C == 4   ? persist_again_c<4, AHEAD>(d, p, x)
+         : d.C == 2 ? persist_again_c<2, AHEAD>(d, p, x)
+                    : persist_again_c<1, AHEAD>(d, p, x);
+}
+
+// Sum over the threads of a segment: a lane's accumulators, then the lanes.
+__device__ __forceinline__ double persist_group_sum(double v, const PersistDir &d) {
+  for (int o = 1; o < d.S; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = d.T >> 1; o >= d.S; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 

@@ -427,33 +427,39 @@ struct PersistArgs {
   int it0, it1;
 };
 
-template <int THREADS, int R>
+// R: elements of a thread's first row and column held in registers, split KR
+// and KC per thread (PersistDir::C); 0: none, any split.
+template <int THREADS, int R, int KR, int KC>
 __global__ void __launch_bounds__(THREADS, 1) k_sirt_persist(const __grid_constant__ PersistArgs a) {
   constexpr int kWarps = THREADS / 32, kAhead = R ? 1 : 2, kParts = 5;  // grids of up to 32 * kParts CTAs
   __shared__ double nrk_sh, sums[kWarps];
   const int gt = blockIdx.x * THREADS + threadIdx.x, total = gridDim.x * THREADS;
-  const int lr = gt % a.rows.L, lc = gt % a.cols.L;
-  const int gr = gt / a.rows.L, gc = gt / a.cols.L;        // first row / column of the group
-  const int nr = total / a.rows.L, nc = total / a.cols.L;  // groups
-  const PersistSeg<R> sr = persist_load<R>(a.rows, gr, lr), sc = persist_load<R>(a.cols, gc, lc);
+  const int lr = gt % a.rows.T, lc = gt % a.cols.T;
+  const int gr = gt / a.rows.T, gc = gt / a.cols.T;        // first row / column of the group
+  const int nr = total / a.rows.T, nc = total / a.cols.T;  // groups
+  const PersistSeg<KR ? KR : 1, R> sr = persist_load<KR ? KR : 1, R>(a.rows, gr, lr);
+  const PersistSeg<KC ? KC : 1, R> sc = persist_load<KC ? KC : 1, R>(a.cols, gc, lc);
   const bool rown = lr == 0 && gr < a.rows.nseg, cown = lc == 0 && gc < a.cols.nseg;
   const double b0 = rown ? a.b[gr] : 0.0, M0 = rown ? a.M[gr] : 0.0, D0 = cown ? a.u.D[gc] : 0.0;
   double x0 = cown ? a.u.x64[gc] : 0.0;
   unsigned target = 0;
-  auto first_dot = [&](const PersistDir &d, const PersistSeg<R> &seg, int i, int lane, const float *x) {
-    return persist_group_sum(R ? persist_dot(d, seg, x) : persist_dot_again<kAhead>(d, i, lane, x), d.L);
+  auto row_sum = [&](int i) {
+    return persist_group_sum(persist_dot_again<KR, kAhead>(a.rows, i, lr, a.u.x32), a.rows);
+  };
+  auto col_sum = [&](int j) {
+    return persist_group_sum(persist_dot_again<KC, kAhead>(a.cols, j, lc, a.mr32), a.cols);
   };
   // r = b - A*x, M.*r and the warps' sums of ||r||^2; thread 0 adds them at
   // the barrier that follows
   auto forward = [&](int it) -> bool {
-    double s = first_dot(a.rows, sr, gr, lr, a.u.x32), r2 = 0.0;
+    double s = R ? persist_group_sum(persist_dot(a.rows, sr, a.u.x32), a.rows) : row_sum(gr), r2 = 0.0;
     if (rown) {
       const double r = b0 - s;
       a.mr32[gr] = (float)(M0 * r);
       r2 = r * r;
     }
     for (int i = gr + nr; !__all_sync(0xffffffffu, i >= a.rows.nseg); i += nr) {
-      s = persist_group_sum(persist_dot_again<kAhead>(a.rows, i, lr, a.u.x32), a.rows.L);
+      s = row_sum(i);
       if (lr == 0 && i < a.rows.nseg) {
         const double r = a.b[i] - s;
         a.mr32[i] = (float)(a.M[i] * r);
@@ -483,7 +489,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_sirt_persist(const __grid_consta
       const int c = threadIdx.x + 32 * q;
       pv[q] = threadIdx.x < 32 && c < (int)gridDim.x ? a.part[(k & 1) * gridDim.x + c] : 0.0;
     }
-    const double s = first_dot(a.cols, sc, gc, lc, a.mr32);
+    const double s = R ? persist_group_sum(persist_dot(a.cols, sc, a.mr32), a.cols) : col_sum(gc);
     if (threadIdx.x < 32) {
       double v = 0.0;
 #pragma unroll
@@ -510,7 +516,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_sirt_persist(const __grid_consta
     const double lam = table ? a.p->relax_table[it - 1] : lam_const;
     if (cown) x0 = update_x_pre(gc, s, lam, a.u, slot, x0, D0);
     for (int j = gc + nc; !__all_sync(0xffffffffu, j >= a.cols.nseg); j += nc) {
-      const double g = persist_group_sum(persist_dot_again<kAhead>(a.cols, j, lc, a.mr32), a.cols.L);
+      const double g = col_sum(j);
       if (lc == 0 && j < a.cols.nseg) update_x_pre(j, g, lam, a.u, slot, a.u.x64[j], a.u.D[j]);
     }
     if (!persist_barrier(a.count, (target += gridDim.x) + a.stall, a.err, a.budget, [] {})) return;
@@ -792,26 +798,45 @@ void launch_bwd(Problem &P, const UpdArgs &u, int relax_kind, const double *Dful
 // Matrices whose iterations run in one launch, and those that are small
 // enough for the variant with part of the matrix in registers.  Per iteration
 // (one launch with registers / without / launched kernels in a graph): 0.16 M
-// nonzeros 6.2 / 9.0 / 12.6 us, 0.94 M 9.2 / 10.8 / 17.4, 1.9 M 15.0 / 14.7 /
-// 20.8, 3.7 M 28 / 21 / 27, 6.3 M 58 / 38.5 / 38.8, 21 M - / 97 / 92.
+// nonzeros 5.3 / 8.4 / 10.7 us, 0.94 M 9.5 / 10.6 / 14.3, 1.9 M 14.5 / 14.9 /
+// 18.6, 3.4 M 24.2 / 23.7 / 23.7, 4.9 M 33.1 / 28.6 / 28.5, 6.3 M 55 / 37.3 /
+// 36.2, 10 M 104 / 54.7 / 52.4.  From 3 to 6 M the last two are level; the one
+// launch has no capture before it and no poll behind it.
 constexpr int64_t kPersistNnz = 6 << 20, kResidentNnz = 7 << 18;
 constexpr int64_t kPersistIters = 2048;  // iterations per launch
 constexpr int kPersistGrid = 160;        // CTAs at most (the kernel adds that many sums)
 
 template <int THREADS, int R>
+auto persist_kernel(int kr, int kc) {
+  if constexpr (R == 0) {
+    return k_sirt_persist<THREADS, 0, 0, 0>;
+  } else {
+    auto of = [&](auto k) {
+      constexpr int K = decltype(k)::value;
+      return kc == 4 ? k_sirt_persist<THREADS, R, K, 4>
+                     : kc == 2 ? k_sirt_persist<THREADS, R, K, 2> : k_sirt_persist<THREADS, R, K, 1>;
+    };
+    return kr == 4   ? of(std::integral_constant<int, 4>{})
+           : kr == 2 ? of(std::integral_constant<int, 2>{})
+                     : of(std::integral_constant<int, 1>{});
+  }
+}
+
+template <int THREADS, int R>
 void run_persist(Problem &P, const FwdOut &fo, const UpdArgs &ua, int64_t kmax) {
   cudaStream_t s = P.stream;
-  auto kernel = k_sirt_persist<THREADS, R>;
   const unsigned grid = (unsigned)std::min(num_sms(), kPersistGrid);
-  auto lanes = [&](int64_t nseg) { return persist_lanes(P.nnz, nseg, (int64_t)grid * THREADS); };
-  int occ = 0;
-  AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, 0));
-  AIRT_REQUIRE(occ >= 1, "the one-launch SIRT kernel cannot be resident");
   P.pst_part.ensure(2 * grid);
   P.pst_count.ensure(1);
   PersistArgs a{};
-  a.rows = PersistDir{(int)P.m, P.rp.p, P.ci.p, P.rv.p, lanes(P.m)};
-  a.cols = PersistDir{(int)P.n, P.cp.p, P.ri.p, P.cv.p, lanes(P.n)};
+  a.rows = PersistDir{(int)P.m, P.rp.p, P.ci.p, P.rv.p};
+  a.cols = PersistDir{(int)P.n, P.cp.p, P.ri.p, P.cv.p};
+  persist_split(a.rows, P.nnz, (int64_t)grid * THREADS);
+  persist_split(a.cols, P.nnz, (int64_t)grid * THREADS);
+  const auto kernel = persist_kernel<THREADS, R>(a.rows.C, a.cols.C);
+  int occ = 0;
+  AIRT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, 0));
+  AIRT_REQUIRE(occ >= 1, "the one-launch SIRT kernel cannot be resident");
   a.b = fo.b;
   a.M = fo.M;
   a.mr32 = fo.mr32;
@@ -1009,7 +1034,7 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
   // a small stored problem runs in one launch (persist.cuh)
   const bool persist = !P.matrix_free && P.spmv_kind == 0 && !me && !dfull && !P.profiling &&
                        o.relax_kind != AIRT_RELAX_LINE && o.kmax < INT32_MAX - 2 && m > 0 && n > 0 && kmax > 0 && P.nnz > 0 &&
-                       P.nnz <= kPersistNnz;
+                       P.nnz <= kPersistNnz && m < (1 << 30) && n < (1 << 30);  // its counters run past the end
   // forward pass, and with NCP the periodogram of the new residual
   const double *Dfull = dfull ? P.Dfull.p : nullptr;
   auto fwd = [&]() {
@@ -1030,7 +1055,9 @@ void run_sirt(Problem &P, const airt_sirt_opts &o, const double *d_b, const doub
     }
   };
   // initial residual and stop check (sirt.m:153-162)
-  if (persist && P.nnz <= kResidentNnz) run_persist<512, 3>(P, fo, ua, kmax);
+  // two lanes per segment may have two elements beside the vectors: not held
+  const bool held = P.nnz <= kResidentNnz && vec_lanes_for(P.nnz, m) > 2 && vec_lanes_for(P.nnz, n) > 2;
+  if (persist && held) run_persist<512, 8>(P, fo, ua, kmax);
   else if (persist) run_persist<1024, 0>(P, fo, ua, kmax);
   else fwd();
 
