@@ -16,6 +16,7 @@
 //    rounding boundary (about one entry in a million) the two differ by one
 //    FP32 unit in the last place.  sphericaltomo and rays the walk refuses are
 //    traced by the tracer of trace.cuh.
+#include <algorithm>
 #include <climits>
 #include <cstring>
 
@@ -515,6 +516,16 @@ void par_prepare(Problem &P) {
     AIRT_CHECK_CUDA(cudaMemcpyAsync(&h, cnt.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
     if (h > kParFixMax) return;
+    // in the order of pixels and rays: the sums of two operators of one
+    // geometry are the same
+    std::vector<ParFix> f(h);
+    if (h) {
+      AIRT_CHECK_CUDA(cudaMemcpyAsync(f.data(), P.par_fix.p, h * sizeof(ParFix), cudaMemcpyDeviceToHost, s));
+      AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+      std::sort(f.begin(), f.end(), [](const ParFix &x, const ParFix &y) { return x.j != y.j ? x.j < y.j : x.r < y.r; });
+      P.par_fix.upload(reinterpret_cast<const double *>(f.data()), 2 * (size_t)h, s);
+      AIRT_CHECK_CUDA(cudaStreamSynchronize(s));
+    }
     P.par_nfix = h;
   }
   P.par_ok = true;

@@ -40,3 +40,16 @@ def test_wide_detectors(p, d):
     a, b = S(u, "transp"), A(u, "transp")
     assert np.all(np.abs(a - b) <= 2.0 ** -23 * np.abs(a) + 1e-8)
     assert p % 2 == 0 or np.any(a > 0)
+
+
+def test_two_operators_of_one_geometry_give_the_same_bits():
+    """Corner pixels that several rays through the corner are corrected at."""
+    N = 30
+    _, p, d, ct, st, off = T.parallel_tables(N, [45.0, 45.0, 135.0, 45.0, 225.0, 45.0, 30.0, 45.0], 43)
+    u = np.random.default_rng(5).uniform(-1.0, 1.0, 8 * 43)
+    first = None
+    for _ in range(6):
+        A = T.parallel_operator(N, ct, st, off, True)
+        v = A(u, "transp")
+        assert first is None or np.array_equal(first, v)
+        first = v
