@@ -19,9 +19,10 @@
 // no work in flight on any stream; where that wait fails (a stream of this
 // thread is capturing) the block is not kept.  The lists are guarded by a
 // mutex.  Kept blocks take at most kKeepBytes and a quarter of the memory that
-// is free beside them (asked once a second), those that nobody asked for
-// during kKeepSeconds go back to the device at the next call, all of them do
-// when an allocation fails and in airt_release_memory.
+// is free beside them (asked once a second): the ones given up first make room
+// for new ones.  Those that nobody asked for during kKeepSeconds go back to
+// the device at the next call, all of them do when an allocation fails and in
+// airt_release_memory.
 #include <cuda.h>
 
 #include <algorithm>
@@ -108,9 +109,11 @@ class BlockPool {
         k.limit = std::min(keep_bytes, be.room() / 4);
         k.asked = t;
       }
-      if (idle && total <= std::max(k.limit, kSmallBytes) && total <= keep_bytes) {
+      const size_t limit = std::min(keep_bytes, std::max(k.limit, kSmallBytes));
+      if (idle && b.size <= limit) {
+        while (k.bytes + b.size > limit) drop_oldest(k);
         k.blocks.insert({b.size, Block{b.p, t}});
-        k.bytes = total;
+        k.bytes += b.size;
         return;
       }
     } catch (...) {  // no host memory for the list
@@ -152,6 +155,16 @@ class BlockPool {
   const size_t keep_bytes;
   std::mutex mu;
   std::map<unsigned long long, Kept> kept;  // by context id
+
+  // Frees the block that was given up first (there is one).
+  void drop_oldest(Kept &k) {
+    auto old = k.blocks.begin();
+    for (auto it = k.blocks.begin(); it != k.blocks.end(); ++it)
+      if (it->second.when < old->second.when) old = it;
+    be.put(old->second.p);
+    k.bytes -= old->first;
+    k.blocks.erase(old);
+  }
 
   // Frees kept blocks of the current context `ctx`: all of them, or (looked
   // at once a second) those unused for long.

@@ -63,6 +63,22 @@ def test_bounds(pool):
     assert p(TAKEN) == 9 * GB
 
 
+def test_the_oldest_blocks_make_room(pool):
+    """A program that turns to other sizes is not left without kept blocks."""
+    p = pool()
+    old = [p(ALLOC, GB) for _ in range(6)]
+    for b in old:
+        p(PASS, 1)
+        p(GIVE, b)
+    for _ in range(3):                          # other sizes, a second later and within one
+        a, b = p(ALLOC, GB // 2), p(ALLOC, GB // 2)
+        p(GIVE, a)
+        p(GIVE, b)
+    assert p(GETS) == 8 and p(PUTS) == 1        # one old block went, the new ones are reused
+    assert p(TAKEN) == 6 * GB
+    assert p(ADDR, p(ALLOC, GB)) != p(ADDR, old[0])
+
+
 def test_old_blocks_go_back(pool):
     p = pool()
     p(GIVE, p(ALLOC, GB))
