@@ -47,9 +47,13 @@ constexpr int kParFixMax = 64;
 // Closed-form chord of a ray at distance d from the pixel centre, as an FP32
 // value in FP64: 0 outside the shadow and for chords within 1e-10 in both
 // coordinates (no entries by the reference's duplicate-point rule).
+__device__ __forceinline__ bool par_entry(double w, double ip, double ipq, double d, double &ramp) {
+  ramp = (w - fabs(d)) * ipq;
+  return ramp > 1e-10 * ip;
+}
 __device__ __forceinline__ double par_chord(double w, double ip, double ipq, double d) {
-  const double ramp = (w - fabs(d)) * ipq;
-  return ramp > 1e-10 * ip ? round24(ramp < ip ? ramp : ip) : 0.0;
+  double ramp;
+  return par_entry(w, ip, ipq, d, ramp) ? round24(ramp < ip ? ramp : ip) : 0.0;
 }
 
 // sum over the angles a0, a0 + da, ... of A(ray, pixel) * u(ray) (u null:
@@ -79,18 +83,17 @@ __device__ __forceinline__ double par_sum(const ParGather &t, const RayGeom &g, 
     double d = fma(kd, t.D, t.s0) - c;
     if (qk.x > 0.0) {
       // at unit spacing two rays at most; without branches their loads and
-      // chords overlap (a chord of 0 is no entry: u may not be finite there)
+      // chords overlap.  u is read where there is an entry, and only there:
+      // it may not be finite beside it
+      auto add = [&] {
+        double ramp;
+        const bool on = par_entry(wi.x, wi.y, qk.x, d, ramp) && k < t.p;
+        const double uk = !on ? 0.0 : u ? (double)__ldg(ua + k) : 1.0;
+        acc = fma(round24(ramp < wi.y ? ramp : wi.y), uk, acc);
+      };
 #pragma unroll
-      for (int q = 0; q < 2; ++q, ++k, d += t.D) {
-        double uk = 0.0;
-        if (d < wi.x && k < t.p) uk = u ? (double)__ldg(ua + k) : 1.0;
-        const double chord = par_chord(wi.x, wi.y, qk.x, d);
-        acc = chord > 0.0 ? fma(chord, uk, acc) : acc;
-      }
-      for (; d < wi.x && k < t.p; ++k, d += t.D) {
-        const double chord = par_chord(wi.x, wi.y, qk.x, d);
-        if (chord > 0.0) acc = fma(chord, u ? (double)__ldg(ua + k) : 1.0, acc);
-      }
+      for (int q = 0; q < 2; ++q, ++k, d += t.D) add();
+      for (; d < wi.x && k < t.p; ++k, d += t.D) add();
     } else {
       // axis-parallel: the pixel holds the rays whose coordinate floors to it
       const bool vert = cs.x != 0.0;  // rays along y at x = c*offset
