@@ -483,6 +483,8 @@ void par_prepare(Problem &P) {
   const double D = (off[P.p - 1] - off[0]) / (P.p - 1);
   // far finer rays than pixels would make a pixel's inner loop long
   if (!(D > 1.0 / 64) || !std::isfinite(D)) return;
+  // ray numbers are taken in 32 bits
+  if (!(std::fabs(off[0]) / D < 1e9)) return;
   // a few ulps of the offsets, but no more than shifts a chord by 1e-9 (a
   // detector of 10^6 pixels or wider: its inner rays are finer than its ends)
   const double tol =

@@ -42,6 +42,14 @@ def test_wide_detectors(p, d):
     assert p % 2 == 0 or np.any(a > 0)
 
 
+@pytest.mark.parametrize("at", [1e6, 2.0 ** 32 - 20, -(2.0 ** 32) - 9, 1e12])
+def test_detectors_far_beside_the_image(at):
+    """No ray meets the image, whatever its distance is in 32 bits."""
+    _, _, _, ct, st, _ = T.parallel_tables(24, [0.0, 30.0, 45.0, 100.0])
+    A = T.parallel_operator(24, ct, st, at + np.arange(30.0), True)
+    assert not np.any(A(np.ones(A.m), "transp")) and not np.any(A(np.ones(A.n), "notransp"))
+
+
 def test_two_operators_of_one_geometry_give_the_same_bits():
     """Corner pixels that several rays through the corner are corrected at."""
     N = 30
