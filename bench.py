@@ -696,7 +696,10 @@ def main():
             traffic, traffic_src = prof[key], prof.get("note")
     except Exception:
         pass
-    launches_per_step = 3 + 1 + 2 + 3 * it   # weights (3), x copy, initial fwd+ctrl, 3/iteration
+    # FP32 copy of x0 and first residual, then transpose + update and residual per
+    # iteration; small problems run in one launch after the copy.  The weights are
+    # kept from the warm-up.
+    launches_per_step = 2 if nnz <= 6 << 20 else 2 + 2 * it
 
     if rank == 0:
         line = {
